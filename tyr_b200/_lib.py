@@ -6,9 +6,10 @@ operator raises, it never routes to PyTorch or to a CPU path.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 
-from .build import LIB_PATH
+from .build import CALLS_PATH, LIB_PATH
 
 c_i32, c_i64, c_u64, c_f32, c_f64, c_u8 = (ctypes.c_int32, ctypes.c_int64, ctypes.c_uint64,
                                            ctypes.c_float, ctypes.c_double, ctypes.c_uint8)
@@ -80,6 +81,7 @@ class BackwardArgs(ctypes.Structure):
 
 
 _lib = None
+_calls = None
 
 
 def load() -> ctypes.CDLL:
@@ -136,6 +138,23 @@ def load() -> ctypes.CDLL:
     L.tyr_b200_attn_launch_count.restype = c_u64
     _lib = L
     return L
+
+
+def calls():
+    """The native call layer (csrc/py_calls.cpp) over the same library; raises if it has not been built."""
+    global _calls
+    if _calls is not None:
+        return _calls
+    import torch  # noqa: F401  (its libraries have to be loaded first)
+    load()
+    if not os.path.exists(CALLS_PATH):
+        raise ImportError(f"{CALLS_PATH} is missing: run `python -c 'import __graft_entry__ as g; g.build()'`")
+    spec = importlib.util.spec_from_file_location("_calls", CALLS_PATH)
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    mod.set_error(AttnError)
+    _calls = mod
+    return mod
 
 
 class AttnError(RuntimeError):

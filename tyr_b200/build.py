@@ -9,6 +9,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libtyr_b200_attn.so")
+CALLS_PATH = os.path.join(LIB_DIR, "_calls.so")   # the Python call layer: a CPython extension over the C ABI
+CALLS_SOURCE = "py_calls.cpp"
 SOURCES = ["api.cu", "prefill_sm100.cu", "backward_sm100.cu", "decode_splitkv.cu", "check_fp32.cu", "qk_prologue.cu",
            "stalled_wait.cu"]
 HEADERS = ["ptx_sm100.cuh", "mma_sync.cuh", "attn_internal.h", os.path.join("..", "..", "include", "tyr_b200_attn.h")]
@@ -30,12 +32,30 @@ def nvcc_path() -> str:
     return nvcc
 
 
-def stale() -> bool:
-    if not os.path.exists(LIB_PATH):
+def _older(path: str, deps) -> bool:
+    if not os.path.exists(path):
         return True
-    t = os.path.getmtime(LIB_PATH)
-    deps = [os.path.join(CSRC, f) for f in SOURCES + HEADERS]
-    return any(os.path.getmtime(d) > t for d in deps)
+    t = os.path.getmtime(path)
+    return any(os.path.getmtime(os.path.join(CSRC, d)) > t for d in deps)
+
+
+def stale() -> bool:
+    return _older(LIB_PATH, SOURCES + HEADERS) or _older(CALLS_PATH, [CALLS_SOURCE, HEADERS[-1]])
+
+
+def _calls_command():
+    """g++ command of the call layer.  It sees the C ABI's header only and is linked against the library next to it."""
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(nvcc_path()))
+    return (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+             f"-I{root}/include", f"-I{root}/include/torch/csrc/api/include", f"-I{cuda}/include",
+             "-I" + sysconfig.get_paths()["include"], os.path.join(CSRC, CALLS_SOURCE), "-o", CALLS_PATH,
+             f"-L{LIB_DIR}", "-l:" + os.path.basename(LIB_PATH), f"-L{root}/lib", "-ltorch_python", "-ltorch", "-ltorch_cpu",
+             "-ltorch_cuda", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"])
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -45,11 +65,12 @@ def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(LIB_DIR, exist_ok=True)
     cmd = [nvcc_path()] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else [])
     cmd += ["-o", LIB_PATH] + [os.path.join(CSRC, f) for f in SOURCES]
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if verbose:
-        print(res.stderr)
-    if res.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + res.stderr)
+    for c in ([cmd] if force or _older(LIB_PATH, SOURCES + HEADERS) else []) + [_calls_command()]:
+        res = subprocess.run(c, capture_output=True, text=True)
+        if verbose:
+            print(res.stderr)
+        if res.returncode != 0:
+            raise RuntimeError(os.path.basename(c[0]) + " failed:\n" + res.stderr)
     return LIB_PATH
 
 

@@ -20,7 +20,7 @@ from typing import Optional, Sequence, Tuple
 import torch
 
 from . import _lib
-from ._lib import AttnError, BackwardArgs, DecodeArgs, PrefillArgs, PrologueArgs, check
+from ._lib import AttnError, PrefillArgs, check
 
 
 def _stream_ptr(t: torch.Tensor) -> int:
@@ -88,37 +88,8 @@ def attentionFwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, is_causal: b
     key-split of a half-empty last round; when the call would split, one is allocated if none is given
     (`workspace=False`: never split).
     """
-    _require_cuda(q, k, v)
-    if q.dim() != 4 or k.dim() != 4 or v.dim() != 4:
-        raise ValueError("q, k, v must be [batch, heads, seq, head_dim]")
-    if out is None:
-        out = torch.empty(q.shape, dtype=q.dtype, device=q.device)
-    if lse is None and return_lse:
-        lse = torch.empty(q.shape[:3], dtype=torch.float32, device=q.device)
-    if lse is not None and (lse.dtype != torch.float32 or not lse.is_contiguous()
-                            or tuple(lse.shape) != tuple(q.shape[:3])):
-        raise ValueError("lse must be a contiguous float32 [batch, n_head, q_seq] tensor")
-    if key_mask is not None:
-        if key_mask.dtype == torch.bool:
-            key_mask = key_mask.view(torch.uint8)
-        if (not key_mask.is_cuda or key_mask.dtype != torch.uint8 or key_mask.dim() != 2
-                or key_mask.stride(1) != 1 or tuple(key_mask.shape) != (k.shape[0], k.shape[2])):
-            raise ValueError("key_mask must be a uint8/bool CUDA tensor [batch, kv_seq]")
-    a = _fill_prefill(q, k, v, out, lse, is_causal, scale, check_mode, window_size, key_mask)
-    L = _lib.load()
-    with torch.cuda.device(q.device):
-        # only unmasked, non-causal calls are ever split: no query for the others
-        may_split = workspace is not False and not is_causal and window_size == 0 and key_mask is None and not check_mode
-        need = int(L.tyr_b200_attn_prefill_workspace_bytes(ctypes.byref(a))) if may_split else 0
-        if need > 0:
-            if workspace is None:
-                workspace = torch.empty(need, dtype=torch.uint8, device=q.device)
-            if (workspace.dtype != torch.uint8 or not workspace.is_contiguous() or workspace.device != q.device
-                    or workspace.data_ptr() % 256 != 0):
-                raise ValueError("workspace must be a contiguous uint8 CUDA tensor on q's device, 256-byte aligned")
-            a.workspace, a.workspace_bytes = workspace.data_ptr(), workspace.numel()
-        check(L.tyr_b200_attn_prefill(ctypes.byref(a), _stream_ptr(q)))
-    return out, lse
+    return _lib.calls().attention_fwd(q, k, v, is_causal, scale, out, lse, return_lse, check_mode, window_size,
+                                      key_mask, workspace)
 
 
 def prefill_workspace_bytes(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, is_causal: bool = True) -> int:
@@ -142,45 +113,7 @@ def attentionBwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Ten
     least `backward_workspace_bytes(...) / 4` elements; one is allocated otherwise.
     `window_size` and `key_mask` are those of the forward call (sliding window / padding keys).
     """
-    _require_cuda(q, k, v, o, d_o, lse)
-    B, Hq, Sq, D = q.shape
-    Bk, Hkv, Skv, Dk = k.shape
-    if (v.shape != k.shape or Bk != B or Dk != D or o.shape != q.shape or d_o.shape != q.shape
-            or tuple(lse.shape) != (B, Hq, Sq)):
-        raise ValueError("shape mismatch among q, k, v, o, d_o, lse")
-    if any(t.dtype != torch.bfloat16 for t in (q, k, v, o, d_o)):
-        raise ValueError("q, k, v, o, d_o must be bfloat16")
-    if lse.dtype != torch.float32 or not lse.is_contiguous():
-        raise ValueError("lse must be a contiguous float32 [batch, n_head, q_seq] tensor")
-    L = _lib.load()
-    need = int(L.tyr_b200_attn_backward_workspace_bytes(B, Hq, Sq))
-    if workspace is None:
-        workspace = torch.empty(need // 4, dtype=torch.float32, device=q.device)
-    if workspace.dtype != torch.float32 or not workspace.is_contiguous() or workspace.numel() * 4 < need:
-        raise ValueError("workspace must be a contiguous float32 CUDA tensor of the required size")
-    d_q, d_k, d_v = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    a = BackwardArgs()
-    a.q, a.k, a.v, a.o, a.d_o, a.lse = (t.data_ptr() for t in (q, k, v, o, d_o, lse))
-    a.d_q, a.d_k, a.d_v = d_q.data_ptr(), d_k.data_ptr(), d_v.data_ptr()
-    a.workspace, a.workspace_bytes = workspace.data_ptr(), workspace.numel() * 4
-    a.batch, a.n_head, a.n_kv_head, a.q_seq, a.kv_seq, a.head_dim = B, Hq, Hkv, Sq, Skv, D
-    for name, t in (("q_stride", q), ("k_stride", k), ("v_stride", v), ("o_stride", o), ("do_stride", d_o),
-                    ("dq_stride", d_q), ("dk_stride", d_k), ("dv_stride", d_v)):
-        getattr(a, name)[:] = [t.stride(0), t.stride(1), t.stride(2)]
-    a.dtype, a.is_causal, a.scale = _lib.TYR_ATTN_BF16, int(bool(is_causal)), float(scale or 0.0)
-    a.window_size = int(window_size)
-    if key_mask is not None:
-        if key_mask.dtype == torch.bool:
-            key_mask = key_mask.view(torch.uint8)
-        if (not key_mask.is_cuda or key_mask.dtype != torch.uint8 or key_mask.dim() != 2
-                or key_mask.stride(1) != 1 or tuple(key_mask.shape) != (B, Skv)):
-            raise ValueError("key_mask must be a uint8/bool CUDA tensor [batch, kv_seq]")
-        a.key_mask, a.key_mask_stride = key_mask.data_ptr(), key_mask.stride(0)
-    else:
-        a.key_mask, a.key_mask_stride = None, 0
-    with torch.cuda.device(q.device):
-        check(L.tyr_b200_attn_backward(ctypes.byref(a), _stream_ptr(q)))
-    return d_q, d_k, d_v
+    return _lib.calls().attention_bwd(q, k, v, o, lse, d_o, is_causal, scale, workspace, window_size, key_mask)
 
 
 def _sdpa(q, k, v, dropout_p, is_causal, enable_gqa):
@@ -236,7 +169,9 @@ def scaledDotProductAttentionGQAMask(query, key, value, attn_mask, dropout_p: fl
         raise AttnError(-2)
     if query.shape[2] != key.shape[2]:
         raise ValueError("scaledDotProductAttentionGQAMask needs q_seq == kv_seq")
-    km = (attn_mask != 0).to(torch.uint8).contiguous()   # one byte per key for the C ABI
+    km = attn_mask        # one byte per key for the C ABI
+    if km.dtype not in (torch.bool, torch.uint8) or km.stride(-1) != 1:
+        km = (km != 0).contiguous()
     out, _ = attentionFwd(query, key, value, is_causal=is_causal, return_lse=False, key_mask=km)
     return out
 
@@ -298,22 +233,13 @@ class DecodePlan:
         self.workspace_bytes = nbytes
 
 
-def _fill_decode(q3, plan: DecodePlan, out, lse, scale) -> DecodeArgs:
-    """Arguments of a ragged decode call over `plan`, without the workspace."""
-    a = DecodeArgs()
-    a.q, a.o, a.lse = q3.data_ptr(), out.data_ptr(), (lse.data_ptr() if lse is not None else None)
-    a.k = a.v = None
-    a.k_ptrs, a.v_ptrs = plan.k_ptrs.data_ptr(), plan.v_ptrs.data_ptr()
-    a.kv_lens, a.kv_head_strides = plan.kv_lens.data_ptr(), plan.head_strides.data_ptr()
-    a.batch, a.n_head, a.n_kv_head = plan.batch, plan.n_head, plan.n_kv_head
-    a.max_kv_seq, a.head_dim = plan.max_kv_seq, plan.head_dim
-    a.q_stride[:] = [q3.stride(0), q3.stride(1)]
-    a.o_stride[:] = [out.stride(0), out.stride(1)]
-    a.k_stride[:] = [0, 0, plan.head_dim]
-    a.v_stride[:] = [0, 0, plan.head_dim]
-    a.scale, a.max_splits = float(scale or 0.0), plan.max_splits
-    a.total_kv_len = plan.total_kv_len     # the host built the plan from these lengths: let the launch size its chunks by them
-    return a
+def _decode_ragged(q, plan: DecodePlan, workspace, scale, out, lse, return_lse):
+    """`workspace` None: the library's own array."""
+    return _lib.calls().decode_ragged(
+        q, plan.batch, plan.n_head, plan.n_kv_head, plan.max_kv_seq, plan.head_dim, plan.max_splits,
+        plan.total_kv_len,     # the host built the plan from these lengths: the launch sizes its chunks by their sum
+        plan.k_ptrs, plan.v_ptrs, plan.kv_lens, plan.head_strides, workspace, plan.workspace_bytes, scale, out, lse,
+        return_lse)
 
 
 def flashDecode(q: torch.Tensor, plan: DecodePlan, scale: Optional[float] = None,
@@ -325,22 +251,7 @@ def flashDecode(q: torch.Tensor, plan: DecodePlan, scale: Optional[float] = None
     scaledDotProductAttentionGQAQKV(q[b:b+1], K_b, V_b, 0.0, false, true) for each b,
     the call QwenAttention.forwardStep makes (Tyr/Model/Qwen/Attention.lean:198-200).
     """
-    squeeze = q.dim() == 4
-    q3 = q[:, :, 0, :] if squeeze else q
-    _require_cuda(q3)
-    if q3.dtype != torch.bfloat16 or q3.shape != (plan.batch, plan.n_head, plan.head_dim):
-        raise ValueError("q must be bf16 [batch, n_head, head_dim]")
-    if out is None:
-        out = torch.empty((plan.batch, plan.n_head, plan.head_dim), dtype=q.dtype, device=q.device)
-    if lse is None and return_lse:
-        lse = torch.empty((plan.batch, plan.n_head), dtype=torch.float32, device=q.device)
-    a = _fill_decode(q3, plan, out, lse, scale)
-    a.workspace, a.workspace_bytes = plan.workspace.data_ptr(), plan.workspace_bytes
-    with torch.cuda.device(q.device):
-        check(_lib.load().tyr_b200_attn_decode(ctypes.byref(a), _stream_ptr(q)))
-    if squeeze:
-        return out.unsqueeze(2), (lse.unsqueeze(2) if lse is not None else None)
-    return out, lse
+    return _decode_ragged(q, plan, plan.workspace, scale, out, lse, return_lse)
 
 
 def flashDecodeStatic(q: torch.Tensor, plan: DecodePlan, scale: Optional[float] = None,
@@ -358,19 +269,7 @@ def flashDecodeStatic(q: torch.Tensor, plan: DecodePlan, scale: Optional[float] 
     The first call on a device looks the array up and should come before any
     stream capture.
     """
-    q3 = q[:, :, 0, :] if q.dim() == 4 else q
-    _require_cuda(q3)
-    if q3.dtype != torch.bfloat16 or q3.shape != (plan.batch, plan.n_head, plan.head_dim):
-        raise ValueError("q must be bf16 [batch, n_head, head_dim]")
-    if out is None:
-        out = torch.empty((plan.batch, plan.n_head, plan.head_dim), dtype=q.dtype, device=q.device)
-    if lse is None:
-        lse = torch.empty((plan.batch, plan.n_head), dtype=torch.float32, device=q.device)
-    a = _fill_decode(q3, plan, out, lse, scale)
-    a.workspace, a.workspace_bytes = None, 0      # ignored: the library's own array is used
-    with torch.cuda.device(q.device):
-        check(_lib.load().tyr_b200_attn_decode_static(ctypes.byref(a), _stream_ptr(q)))
-    return out, lse
+    return _decode_ragged(q, plan, None, scale, out, lse, True)
 
 
 def flashDecodeDense(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
@@ -380,32 +279,7 @@ def flashDecodeDense(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
     """Decode over Tyr's dense KVCache layout [batch, n_kv_head, cap, head_dim]
     (Tyr/Model/Qwen/Attention.lean:54-68).  `kv_len` plays the cache's shared `seq`
     counter; `kv_lens` (int32 device tensor) makes it per sequence."""
-    _require_cuda(q, k_cache, v_cache)
-    B, Hq, D = q.shape[0], q.shape[1], q.shape[-1]
-    q3 = q[:, :, 0, :] if q.dim() == 4 else q
-    max_len = int(kv_len if kv_len is not None else k_cache.shape[2])
-    out = torch.empty((B, Hq, D), dtype=q.dtype, device=q.device)
-    lse = torch.empty((B, Hq), dtype=torch.float32, device=q.device)
-    L = _lib.load()
-    nbytes = L.tyr_b200_attn_decode_workspace_bytes(B, Hq, D, max_len, max_splits)
-    if workspace is None:
-        workspace = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=q.device)
-    a = DecodeArgs()
-    a.q, a.o, a.lse = q3.data_ptr(), out.data_ptr(), lse.data_ptr()
-    a.k, a.v = k_cache.data_ptr(), v_cache.data_ptr()
-    a.k_ptrs = a.v_ptrs = a.kv_head_strides = None
-    a.kv_lens = kv_lens.data_ptr() if kv_lens is not None else None
-    a.batch, a.n_head, a.n_kv_head, a.max_kv_seq, a.head_dim = B, Hq, k_cache.shape[1], max_len, D
-    a.q_stride[:] = [q3.stride(0), q3.stride(1)]
-    a.o_stride[:] = [out.stride(0), out.stride(1)]
-    a.k_stride[:] = [k_cache.stride(0), k_cache.stride(1), k_cache.stride(2)]
-    a.v_stride[:] = [v_cache.stride(0), v_cache.stride(1), v_cache.stride(2)]
-    a.scale, a.max_splits = float(scale or 0.0), max_splits
-    a.total_kv_len = 0                     # a shared length is known as it is; per-sequence lengths live on the device
-    a.workspace, a.workspace_bytes = workspace.data_ptr(), workspace.numel()
-    with torch.cuda.device(q.device):
-        check(L.tyr_b200_attn_decode(ctypes.byref(a), _stream_ptr(q)))
-    return out, lse
+    return _lib.calls().decode_dense(q, k_cache, v_cache, kv_lens, kv_len, scale, workspace, max_splits)
 
 
 def qkPrologue(x: torch.Tensor, out: torch.Tensor, norm_weight: Optional[torch.Tensor] = None,
@@ -428,48 +302,7 @@ def qkPrologue(x: torch.Tensor, out: torch.Tensor, norm_weight: Optional[torch.T
     position is known on the host (position0); with device-side `positions` the kernel skips
     them and sets the out-of-range bit of the device status word.
     """
-    _require_cuda(x, out)
-    if x.dim() != 4 or out.dim() != 4 or x.dtype != torch.bfloat16 or out.dtype != torch.bfloat16:
-        raise ValueError("x must be bf16 [B,S,H,D] and out bf16 [B,H,cap,D]")
-    B, S, H, D = x.shape
-    if out.shape[0] != B or out.shape[1] != H or out.shape[3] != D:
-        raise ValueError("out does not match x")
-    for t_ in (norm_weight, cos, sin, pe):
-        if t_ is not None and (t_.dtype != torch.float32 or not t_.is_contiguous() or not t_.is_cuda):
-            raise ValueError("norm_weight / cos / sin / pe must be contiguous float32 CUDA tensors")
-    if pe is not None:
-        if cos is not None or sin is not None:
-            raise ValueError("pass either cos/sin or pe")
-        if pe.dim() != 5 or tuple(pe.shape[2:]) != (D // 2, 2, 2) or pe.shape[0] not in (1, B):
-            raise ValueError("pe must be [B or 1, max_pos, D/2, 2, 2]")
-    cap = out.shape[2]
-    max_pos = pe.shape[1] if pe is not None else (cos.shape[0] if cos is not None else 0)
-    if cos is not None and (sin is None or tuple(cos.shape) != tuple(sin.shape) or cos.dim() != 2 or cos.shape[1] != D // 2):
-        raise ValueError("cos and sin must both be [max_pos, D/2]")
-    if out_at_row0 and S > cap:
-        raise ValueError(f"{S} rows do not fit the {cap} rows of out")
-    if positions is None:
-        if position0 < 0 or (not out_at_row0 and position0 + S > cap):
-            raise ValueError(f"rows {position0}..{position0 + S - 1} do not fit the {cap} rows of out")
-        if max_pos and position0 + S > max_pos:
-            raise ValueError(f"positions up to {position0 + S - 1} exceed the {max_pos} rows of the rotary table")
-    if positions is not None and (positions.dtype != torch.int32 or not positions.is_cuda):
-        raise ValueError("positions must be an int32 CUDA tensor")
-    a = PrologueArgs()
-    a.x, a.out = x.data_ptr(), out.data_ptr()
-    a.norm_weight = norm_weight.data_ptr() if norm_weight is not None else None
-    a.cos = cos.data_ptr() if cos is not None else None
-    a.sin = sin.data_ptr() if sin is not None else None
-    a.positions = positions.data_ptr() if positions is not None else None
-    a.position0, a.batch, a.seq, a.n_head, a.head_dim = int(position0), B, S, H, D
-    a.x_stride[:] = [x.stride(0), x.stride(1), x.stride(2)]
-    a.out_stride[:] = [out.stride(0), out.stride(1), out.stride(2)]
-    a.eps = float(eps)
-    a.cap, a.max_pos, a.out_at_row0 = int(cap), int(max_pos), int(bool(out_at_row0))
-    a.pe = pe.data_ptr() if pe is not None else None
-    a.pe_batch_stride = pe.stride(0) if (pe is not None and pe.shape[0] > 1) else 0
-    with torch.cuda.device(x.device):
-        check(_lib.load().tyr_b200_attn_qk_prologue(ctypes.byref(a), _stream_ptr(x)))
+    _lib.calls().qk_prologue(x, out, norm_weight, cos, sin, positions, position0, eps, pe, out_at_row0)
     return out
 
 
