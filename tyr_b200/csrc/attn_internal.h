@@ -8,6 +8,34 @@
 
 namespace tyr {
 
+// Launch with programmatic stream serialisation: the kernel's CTAs may become resident while the
+// grid before it in the stream is still draining.  Every kernel launched this way executes
+// griddepcontrol.wait (grid_dependency_wait) in every thread block before it touches memory that an
+// earlier grid may write or still read, so only its launch latency and set-up overlap.  A grid lets
+// its successor start by griddepcontrol.launch_dependents (grid_launch_dependents).
+template <class... P, class... A>
+inline cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, unsigned cluster_x,
+                                     A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cluster_x > 1) {
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster_x;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
+  }
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Per-device state owned by api.cu.
 struct DeviceState {
   int* status = nullptr;  // device word the kernels' bounded waits OR into
@@ -38,6 +66,10 @@ int launch_prefill_check(const TyrAttnPrefillArgs& a, float scale, cudaStream_t 
 size_t decode_workspace_bytes(int batch, int n_head, int head_dim, int max_kv_seq, int max_splits);
 int decode_num_splits(int max_kv_seq, int max_splits, int* chunk_len);
 int launch_decode(const TyrAttnDecodeArgs& a, float scale, cudaStream_t st);
+// Unmasked forward calls with few query rows per KV head (group * q_seq), served by the decode kernel.
+bool few_rows_call(const TyrAttnPrefillArgs& a);
+size_t few_rows_workspace_bytes(const TyrAttnPrefillArgs& a);  // 0: the launch would not use one
+int launch_few_rows(const TyrAttnPrefillArgs& a, float scale, int* status, cudaStream_t st);
 int launch_merge2(const float* o_a, const float* lse_a, const float* o_b, const float* lse_b,
                   float* o_out, float* lse_out, int64_t rows, int head_dim, cudaStream_t st);
 
