@@ -1,0 +1,68 @@
+"""The cuts of the decode kernel's keys (cluster merge, one chunk, workspace) and the few-row typed call, against the oracle."""
+import numpy as np
+import pytest
+import torch
+
+from conftest import LSE_REL, O_MAX_ABS
+from oracle import c_oracle
+from tyr_b200 import nn as tnn
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def randn(*shape, seed=0):
+    g = torch.Generator(device="cpu").manual_seed(seed)
+    return torch.randn(*shape, generator=g).bfloat16()
+
+
+def check(o, lse, q, k, v):
+    ro, rl = c_oracle.sdpa(q.float().numpy(), k.float().numpy(), v.float().numpy(), False)
+    assert np.abs(o.float().cpu().numpy() - ro).max() <= O_MAX_ABS
+    if lse is not None:
+        assert (np.abs(lse.cpu().numpy() - rl) / np.maximum(np.abs(rl), 1.0)).max() <= LSE_REL
+
+
+@pytest.fixture(autouse=True)
+def _status_clean():
+    yield
+    assert tnn.device_status(0, True) == 0
+
+
+# clusters of 16, 8, 7, 5, 2 CTAs, CTAs without keys, one chunk per sequence (8 and 4 warps), more than 8 query rows per
+# KV head, and the workspace form next to them
+@pytest.mark.parametrize("B,Hq,Hkv,L", [(1, 8, 2, 1), (1, 8, 2, 65), (1, 8, 8, 1025), (4, 8, 8, 515), (4, 36, 9, 700), (3, 16, 16, 640),
+                                        (7, 16, 16, 131), (9, 16, 16, 90), (20, 16, 16, 77), (1, 40, 2, 300), (2, 24, 2, 2000),
+                                        (1, 4, 1, 20000), (3, 48, 48, 1100)])
+@pytest.mark.parametrize("D", [64, 128])
+def test_dense_decode(B, Hq, Hkv, L, D):
+    q, k, v = randn(B, Hq, 1, D, seed=L), randn(B, Hkv, L, D, seed=L + 1), randn(B, Hkv, L, D, seed=L + 2)
+    o, lse = tnn.flashDecodeDense(q.to(DEV), k.to(DEV), v.to(DEV))
+    check(o[:, :, None], lse[:, :, None], q, k, v)
+    o = tnn.scaledDotProductAttentionGQAQKV(q.to(DEV), k.to(DEV), v.to(DEV), 0.0, False, True)
+    check(o, None, q, k, v)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_clusters_over_ragged_lengths(D):
+    # lengths on the device: some CTAs of a short sequence's cluster find no keys
+    lens, cap = [1, 16, 17, 200, 513, 900], 900
+    k, v, q = randn(6, 4, cap, D, seed=1), randn(6, 4, cap, D, seed=2), randn(6, 16, 1, D, seed=3)
+    for b, n in enumerate(lens):
+        k[b, :, n:] = float("nan")
+        v[b, :, n:] = float("nan")
+    dl = torch.tensor(lens, dtype=torch.int32, device=DEV)
+    o, lse = tnn.flashDecodeDense(q.to(DEV), k.to(DEV), v.to(DEV), kv_lens=dl)
+    for b, n in enumerate(lens):
+        check(o[b:b + 1, :, None], lse[b:b + 1, :, None], q[b:b + 1], k[b:b + 1, :, :n], v[b:b + 1, :, :n])
+
+
+# group * q_seq at and around the 8-column tiles and the limit of 16 rows; 17 rows go to the tensor-core kernel
+@pytest.mark.parametrize("Hq,Hkv,Sq", [(2, 2, 7), (2, 2, 8), (2, 2, 9), (4, 2, 8), (2, 2, 16), (2, 2, 17), (6, 2, 5)])
+@pytest.mark.parametrize("workspace", [None, False])
+def test_few_query_rows(Hq, Hkv, Sq, workspace):
+    D, L = 128, 1500
+    q, k, v = randn(2, Sq, Hq, D, seed=Sq).transpose(1, 2), randn(2, Hkv, L, D, seed=5), randn(2, Hkv, L, D, seed=6)
+    buf = torch.full((2, Sq, Hq, D), 7.0, dtype=torch.bfloat16, device=DEV)     # [B,S,H,D] storage on both sides
+    o, lse = tnn.attentionFwd(q.to(DEV), k.to(DEV), v.to(DEV), is_causal=False, out=buf.transpose(1, 2), workspace=workspace)
+    check(o, lse, q, k, v)

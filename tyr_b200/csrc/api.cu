@@ -203,6 +203,7 @@ int tyr_b200_attn_prefill(const TyrAttnPrefillArgs* a, void* stream) {
   if ((rc = current_device_checked(&dev))) return rc;
   DeviceState* ds = device_state(dev);
   if (!ds) return -TYR_ATTN_ERR_NO_DEVICE;
+  if (few_rows_call(*a)) return launch_few_rows(*a, scale, ds->status, st);
   return launch_prefill_sm100(*a, scale, ds->status, st);
 }
 
@@ -373,6 +374,7 @@ int64_t tyr_b200_attn_prefill_workspace_bytes(const TyrAttnPrefillArgs* a) {
   const int rc = check_prefill(a);
   if (rc) return rc;
   if (a->dtype != TYR_ATTN_BF16 || a->check_mode) return 0;
+  if (few_rows_call(*a)) return (int64_t)few_rows_workspace_bytes(*a);
   return tyr::prefill_split_workspace_bytes(*a);
 }
 

@@ -7,14 +7,27 @@
 // from HBM exactly once: one CTA owns (sequence, KV head, chunk of keys) and
 // serves all query heads of that KV head together.  The merge is the formula of
 // ringAttnReduce (Tyr/GPU/Kernels/RingAttn.lean:164-180), kept in the log2 domain.
+// It runs in one of two places: in the launch itself, when the CTAs that share a sequence and KV head
+// form a cluster and exchange their partials through distributed shared memory (small launches), or
+// in a second launch over partials in the workspace.
+//
+// A call with a few query rows per head (the typed call of a generating loop, q_seq = 1, and other
+// unmasked calls with group * q_seq <= kMaxFewRows) is served by the same kernel: the rows of a KV head
+// are its (query head, query row) pairs.
 //
 // The kernel is HBM-bound.  Keys stream global -> shared with 16-byte cp.async
 // into a 3-stage ring (XOR-swizzled rows, conflict-free for ldmatrix); the tiny
 // contractions (<=16 query rows) run on warp-level m16n8k16 MMAs so that issue
-// slots stay free for the loads.  Each warp owns 16 of the 64 keys of a stage and
-// keeps its own (max, sum, O); the four warps merge through shared memory.
+// slots stay free for the loads.  Each warp owns 16 of the keys of a stage and
+// keeps its own (max, sum, O); the warps merge through shared memory.
+// Both products are formed transposed, keys (S^T = K Q^T) and head dims (O^T = V^T P^T) as the 16
+// rows of the MMA and query rows as its 8 columns: a warp-level MMA takes about 31 cycles of its SM
+// sub-partition here whatever it is used for, and with the up to 8 query rows of a usual group in the
+// 16-row operand half of each was wasted.
 #include <cuda_bf16.h>
 
+#include <algorithm>
+#include <atomic>
 #include <mutex>
 
 #include "attn_internal.h"
@@ -24,9 +37,10 @@
 namespace tyr {
 namespace {
 
-constexpr int kThreads = 128;
-constexpr int kTileKeys = 64;   // keys per pipeline stage
+constexpr int kWarpKeys = 16;   // keys of a pipeline stage one warp works on
 constexpr int kStages = 3;
+constexpr int kMergeThreads = 128;
+constexpr int kMaxFewRows = 16;
 constexpr int kMinChunk = 256;  // keys; shorter chunks only add merge traffic
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
@@ -40,73 +54,93 @@ struct DecodeParams {
   const void* const* v_ptrs;
   const int32_t* kv_lens;
   const int64_t* kv_head_strides;
-  int batch, n_head, n_kv_head, max_kv_seq, group, head_groups;
-  int64_t qs[2], os[2], ks[3], vs[3];
+  int batch, n_head, n_kv_head, max_kv_seq;
+  int q_seq;        // query rows per head (1 in the decode entries)
+  int rows;         // query rows per KV head: group * q_seq, row r = (head r / q_seq of the group, query r % q_seq)
+  int row_groups;   // CTAs (of up to 16 rows each) per KV head and chunk of keys
+  int64_t qs[3], os[3], ks[3], vs[3];  // qs, os: batch, head, query row
   float scale_log2;
   int chunk_len, n_splits;
-  float* ws_o;    // [batch, n_head, n_splits, D] normalised partial outputs
-  float* ws_lse;  // [batch, n_head, n_splits] log2-domain partial LSE
+  float* ws_o;    // [batch, n_head * q_seq, n_splits, D] normalised partial outputs
+  float* ws_lse;  // [batch, n_head * q_seq, n_splits] log2-domain partial LSE
+  int ws_aligned; // ws_o is 16-byte aligned
   int* status;    // per-device status word (out-of-range lengths are reported there)
 };
+
+// Row `r` of the KV head's rows (query head and query row) in O and in the LSE array.
+__device__ __forceinline__ __nv_bfloat16* o_row(const DecodeParams& p, int b, int hkv, int r) {
+  const int h = r / p.q_seq, i = r - h * p.q_seq;
+  return p.o + b * p.os[0] + (int64_t)(hkv * (p.rows / p.q_seq) + h) * p.os[1] + i * p.os[2];
+}
+__device__ __forceinline__ int64_t lse_index(const DecodeParams& p, int b, int hkv, int r) {
+  return (int64_t)b * p.n_head * p.q_seq + hkv * p.rows + r;
+}
 
 // A length outside [1, max_kv_seq] (the workspace and the grid are sized for max_kv_seq, so a
 // longer one would index past both): report it once per sequence, give a sequence without any
 // key a defined row (zeros, LSE = -inf), and return the length forced into [0, max_kv_seq].
 // Kept out of line so that this rare path costs the scan loop no registers.
 template <int D>
-__device__ __noinline__ int bad_length(int raw, int max_kv_seq, bool first_cta_of_row, int* status,
-                                       __nv_bfloat16* o_row0, int64_t o_head_stride, float* lse_row0,
-                                       int head0, int heads_here) {
-  const int len = min(max(raw, 0), max_kv_seq);
-  if (first_cta_of_row) {
-    if (threadIdx.x == 0 && head0 == 0) atomicOr(status, kStatusOutOfRange);
+__device__ __noinline__ int bad_length(int raw, const DecodeParams& p, int b, int hkv, int row0, int rows_here) {
+  const int len = min(max(raw, 0), p.max_kv_seq);
+  if (blockIdx.x == 0) {
+    if (threadIdx.x == 0 && hkv == 0 && row0 == 0) atomicOr(p.status, kStatusOutOfRange);
     if (len == 0) {
-      for (int idx = threadIdx.x; idx < heads_here * D; idx += blockDim.x) {
-        const int head = head0 + idx / D, d = idx % D;
-        o_row0[(int64_t)head * o_head_stride + d] = __float2bfloat16_rn(0.f);
-        if (d == 0 && lse_row0) lse_row0[head] = -INFINITY;
+      for (int idx = threadIdx.x; idx < rows_here * D; idx += blockDim.x) {
+        const int r = row0 + idx / D, d = idx % D;
+        o_row(p, b, hkv, r)[d] = __float2bfloat16_rn(0.f);
+        if (d == 0 && p.lse) p.lse[lse_index(p, b, hkv, r)] = -INFINITY;
       }
     }
   }
   return len;
 }
 
-template <int D>
+template <int D, int kWarps, int kNT>
 struct DCfg {
+  static constexpr int kRows = 8 * kNT;                 // query rows of a CTA, in column tiles of 8
+  static constexpr int kThreads = 32 * kWarps;
+  static constexpr int kTileKeys = kWarpKeys * kWarps;  // keys per pipeline stage
   static constexpr int kRowBytes = D * 2;
   static constexpr int kChunksPerRow = D / 8;  // 16-byte chunks
   static constexpr int kTileBytes = kTileKeys * kRowBytes;
   static constexpr int kStageBytes = 2 * kTileBytes;  // K then V
   static constexpr int kSmemBytes = kStages * kStageBytes;
-  // cross-warp merge reuses the ring: 4 warps x 16 rows of D floats, rows padded by 4 floats so that
-  // the eight rows a warp stores at once fall on different banks, + 2 floats of (max, sum) per row
+  // cross-warp merge reuses the ring: the warps' rows of D floats, rows padded by 4 floats so that
+  // the pieces of four rows a warp stores at once fall on different banks, + 2 floats of (max, sum) per row
   static constexpr int kMergeStride = D + 4;
-  static_assert(4 * 16 * (kMergeStride + 2) * 4 <= kSmemBytes, "merge scratch fits in the ring");
+  // ... and behind it, for a cluster's merge, this CTA's rows of D floats and their (max, sum)
+  static constexpr int kPartOff = kWarps * kRows * (kMergeStride + 2);  // in floats
+  static_assert((kPartOff + kRows * (D + 2)) * 4 <= kSmemBytes, "merge scratch fits in the ring");
 };
 
-template <int D>
-__global__ void __launch_bounds__(kThreads)
-decode_kernel(const DecodeParams p) {
-  using C = DCfg<D>;
+// kCluster: the grid's x extent is one cluster, its CTAs cut the sequence's keys evenly and merge among
+// themselves; no workspace, no second launch.  Otherwise chunks of p.chunk_len keys, partials to the workspace.
+template <int D, int kWarps, int kNT, bool kCluster>
+__global__ void __launch_bounds__(32 * kWarps)
+decode_kernel(const __grid_constant__ DecodeParams p) {
+  using C = DCfg<D, kWarps, kNT>;
+  constexpr int kThreads = C::kThreads, kTileKeys = C::kTileKeys, kRows = C::kRows;
   extern __shared__ __align__(128) uint8_t smem[];
   const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
 
-  // the merge kernel behind this one may start to become resident (it waits for this grid itself)
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  grid_launch_dependents();
+  grid_dependency_wait();
   const int split = blockIdx.x;
-  const int hkv = blockIdx.y / p.head_groups;
-  const int hg = blockIdx.y % p.head_groups;
+  const int hkv = blockIdx.y / p.row_groups;
+  const int row0 = (blockIdx.y % p.row_groups) * kRows;   // first of the KV head's rows this CTA serves
+  const int rows_here = min(kRows, p.rows - row0);
   const int b = blockIdx.z;
   int len = p.kv_lens ? p.kv_lens[b] : p.max_kv_seq;
-  if (len <= 0 || len > p.max_kv_seq)
-    len = bad_length<D>(len, p.max_kv_seq, split == 0, p.status, p.o + b * p.os[0], p.os[1],
-                        p.lse ? p.lse + (int64_t)b * p.n_head : nullptr, hkv * p.group + hg * 16,
-                        min(16, p.group - hg * 16));
-  const int n_chunks = (len + p.chunk_len - 1) / p.chunk_len;
-  if (split >= n_chunks) return;
-  const int key_begin = split * p.chunk_len;
-  const int key_end = min(len, key_begin + p.chunk_len);
-  const int n_tiles = (key_end - key_begin + kTileKeys - 1) / kTileKeys;
+  if (len <= 0 || len > p.max_kv_seq) len = bad_length<D>(len, p, b, hkv, row0, rows_here);
+  if (kCluster && len == 0) return;  // the whole cluster: its CTAs share the sequence
+  int chunk_len = p.chunk_len;
+  if (kCluster) chunk_len = ((len + p.n_splits - 1) / p.n_splits + kWarpKeys - 1) / kWarpKeys * kWarpKeys;
+  const int n_chunks = (len + chunk_len - 1) / chunk_len;
+  if (!kCluster && split >= n_chunks) return;
+  const int key_begin = split * chunk_len;
+  const int key_end = min(len, key_begin + chunk_len);
+  const int n_tiles = max(key_end - key_begin + kTileKeys - 1, 0) / kTileKeys;  // 0: a CTA of the cluster without keys
 
   const __nv_bfloat16 *kbase, *vbase;
   if (p.k_ptrs) {
@@ -136,42 +170,37 @@ decode_kernel(const DecodeParams p) {
     }
   };
 
-  // ---- Q fragments (A operand, 16 rows = query heads of this KV head)
-  const int head0 = hkv * p.group + hg * 16;       // first query head of this CTA
-  const int heads_here = min(16, p.group - hg * 16);
-  uint32_t qa[D / 16][4];
-  {
-    const __nv_bfloat16* qb = p.q + b * p.qs[0];
-#pragma unroll
-    for (int ks = 0; ks < D / 16; ++ks) {
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {      // rows quad, quad + 8
-        const int r = quad + half * 8;
-#pragma unroll
-        for (int kh = 0; kh < 2; ++kh) {          // d, d + 8
-          uint32_t val = 0;
-          if (r < heads_here)
-            val = *reinterpret_cast<const uint32_t*>(qb + (int64_t)(head0 + r) * p.qs[1] + ks * 16 +
-                                                     kh * 8 + t4 * 2);
-          qa[ks][half + 2 * kh] = val;
-        }
-      }
-    }
-  }
-
 #pragma unroll
   for (int s = 0; s < kStages - 1; ++s) {
     if (s < n_tiles) load_tile(s, s);
     cp_async_commit();
   }
 
-  float m_run[2] = {-INFINITY, -INFINITY};  // rows quad, quad + 8 (log2 domain)
-  float l_run[2] = {0.f, 0.f};
-  float oacc[D / 8][4];
+  // ---- Q fragments (B operand: column = query row of this KV head)
+  uint32_t qb[kNT][D / 16][2];
 #pragma unroll
-  for (int n = 0; n < D / 8; ++n)
+  for (int nt = 0; nt < kNT; ++nt) {
+    const int r = row0 + nt * 8 + quad, h = r / p.q_seq;
+    const bool live = nt * 8 + quad < rows_here;
+    const __nv_bfloat16* qr = p.q + b * p.qs[0] + (int64_t)(hkv * (p.rows / p.q_seq) + h) * p.qs[1] + (r - h * p.q_seq) * p.qs[2];
 #pragma unroll
-    for (int x = 0; x < 4; ++x) oacc[n][x] = 0.f;
+    for (int ks = 0; ks < D / 16; ++ks)
+#pragma unroll
+      for (int kh = 0; kh < 2; ++kh)          // d, d + 8
+        qb[nt][ks][kh] = live ? *reinterpret_cast<const uint32_t*>(qr + ks * 16 + kh * 8 + t4 * 2) : 0u;
+  }
+
+  float m_run[kNT][2], l_run[kNT][2];  // query rows nt * 8 + 2 t4, + 1 (log2 domain; l: this lane's keys only)
+  float oacc[kNT][D / 16][4];          // O^T: dims 16 m + quad (+ 8 in [2], [3]), the same two query rows
+#pragma unroll
+  for (int nt = 0; nt < kNT; ++nt) {
+    m_run[nt][0] = m_run[nt][1] = -INFINITY;
+    l_run[nt][0] = l_run[nt][1] = 0.f;
+#pragma unroll
+    for (int m = 0; m < D / 16; ++m)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) oacc[nt][m][x] = 0.f;
+  }
 
   for (int tile = 0; tile < n_tiles; ++tile) {
     cp_async_wait<kStages - 2>();
@@ -181,151 +210,252 @@ decode_kernel(const DecodeParams p) {
 
     const int stage = tile % kStages;
     const uint32_t sk = sbase + stage * C::kStageBytes, sv = sk + C::kTileBytes;
-    const int wkey0 = warp * 16;                              // this warp's keys in the tile
+    const int wkey0 = warp * kWarpKeys;                              // this warp's keys in the tile
     const int gkey0 = key_begin + tile * kTileKeys + wkey0;   // global index of the first
     if (gkey0 >= key_end) continue;                           // warp-uniform: nothing valid
 
-    // S = Q K^T for 16 keys: two n-tiles of 8 keys
-    float sacc[2][4];
+    // S^T = K Q^T for 16 keys, as two chains over alternate 16-element groups of the head dimension
+    // (an MMA's result is some 30 cycles away from the next one's input)
+    float sacc[kNT][2][4];
 #pragma unroll
-    for (int n = 0; n < 2; ++n)
+    for (int nt = 0; nt < kNT; ++nt)
 #pragma unroll
-      for (int x = 0; x < 4; ++x) sacc[n][x] = 0.f;
+      for (int x = 0; x < 8; ++x) sacc[nt][x >> 2][x & 3] = 0.f;
 #pragma unroll
-    for (int n = 0; n < 2; ++n) {
+    for (int ks = 0; ks < D / 16; ++ks) {
+      uint32_t ka[4];
+      ldsm_x4(sk + sw_off<D>(wkey0 + (lane & 15), 2 * ks + (lane >> 4)), ka);
 #pragma unroll
-      for (int c = 0; c < C::kChunksPerRow; c += 4) {
-        uint32_t kb[4];
-        ldsm_x4(sk + sw_off<D>(wkey0 + n * 8 + (lane & 7), c + (lane >> 3)), kb);
-        mma_bf16_16816(sacc[n], qa[c / 2], kb[0], kb[1]);
-        mma_bf16_16816(sacc[n], qa[c / 2 + 1], kb[2], kb[3]);
+      for (int nt = 0; nt < kNT; ++nt) mma_bf16_16816(sacc[nt][ks & 1], ka, qb[nt][ks][0], qb[nt][ks][1]);
+    }
+    // scale, mask the tail, online softmax per query row; this lane has keys quad and quad + 8
+    const bool live0 = gkey0 + quad < key_end, live1 = gkey0 + quad + 8 < key_end;
+    float sx[kNT][4], mx[kNT][2];
+    bool grown = false;
+#pragma unroll
+    for (int nt = 0; nt < kNT; ++nt)
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        sx[nt][x] = live0 ? (sacc[nt][0][x] + sacc[nt][1][x]) * p.scale_log2 : -INFINITY;
+        sx[nt][2 + x] = live1 ? (sacc[nt][0][2 + x] + sacc[nt][1][2 + x]) * p.scale_log2 : -INFINITY;
+        mx[nt][x] = fmaxf(sx[nt][x], sx[nt][2 + x]);
+      }
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1)
+#pragma unroll
+      for (int nt = 0; nt < kNT; ++nt)
+#pragma unroll
+        for (int x = 0; x < 2; ++x) mx[nt][x] = fmaxf(mx[nt][x], __shfl_xor_sync(0xffffffffu, mx[nt][x], o));
+#pragma unroll
+    for (int nt = 0; nt < kNT; ++nt)
+#pragma unroll
+      for (int x = 0; x < 2; ++x) grown = grown || mx[nt][x] > m_run[nt][x];
+    if (__any_sync(0xffffffffu, grown)) {  // after the first tiles a row's maximum seldom moves
+#pragma unroll
+      for (int nt = 0; nt < kNT; ++nt) {
+        float alpha[2];
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          const float m_new = fmaxf(m_run[nt][x], mx[nt][x]);  // finite: key gkey0 is valid
+          alpha[x] = ex2f(m_run[nt][x] - m_new);               // 0 on the first tile
+          m_run[nt][x] = m_new;
+          l_run[nt][x] *= alpha[x];
+        }
+#pragma unroll
+        for (int m = 0; m < D / 16; ++m) {
+          oacc[nt][m][0] *= alpha[0];
+          oacc[nt][m][1] *= alpha[1];
+          oacc[nt][m][2] *= alpha[0];
+          oacc[nt][m][3] *= alpha[1];
+        }
       }
     }
-    // scale, mask the tail, online softmax per row (rows quad and quad+8)
-    float mx[2] = {-INFINITY, -INFINITY};
+    // P^T as the B operand: the 8 x 8 blocks (keys x query rows) are transposed between the lanes
+    uint32_t pb[kNT][2];
 #pragma unroll
-    for (int n = 0; n < 2; ++n)
-#pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        const int key = gkey0 + n * 8 + t4 * 2 + (x & 1);
-        const float sv2 = (key < key_end) ? sacc[n][x] * p.scale_log2 : -INFINITY;
-        sacc[n][x] = sv2;
-        mx[x >> 1] = fmaxf(mx[x >> 1], sv2);
-      }
-    float alpha[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
-      mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
-      const float m_new = fmaxf(m_run[h], mx[h]);  // finite: key gkey0 is valid
-      alpha[h] = ex2f(m_run[h] - m_new);           // 0 on the first tile
-      m_run[h] = m_new;
+    for (int nt = 0; nt < kNT; ++nt) {
+      const float p0 = ex2f(sx[nt][0] - m_run[nt][0]), p1 = ex2f(sx[nt][1] - m_run[nt][1]);
+      const float p2 = ex2f(sx[nt][2] - m_run[nt][0]), p3 = ex2f(sx[nt][3] - m_run[nt][1]);
+      l_run[nt][0] += p0 + p2;
+      l_run[nt][1] += p1 + p3;
+      pb[nt][0] = transpose_8x8(pack2(p0, p1));
+      pb[nt][1] = transpose_8x8(pack2(p2, p3));
     }
-    float ps[2] = {0.f, 0.f};
-    uint32_t pa[4];
+    // O^T += V^T P^T : k = this warp's 16 keys, m-tiles of 16 output dims
 #pragma unroll
-    for (int n = 0; n < 2; ++n) {
-      const float p0 = ex2f(sacc[n][0] - m_run[0]), p1 = ex2f(sacc[n][1] - m_run[0]);
-      const float p2 = ex2f(sacc[n][2] - m_run[1]), p3 = ex2f(sacc[n][3] - m_run[1]);
-      ps[0] += p0 + p1;
-      ps[1] += p2 + p3;
-      pa[2 * n] = pack2(p0, p1);      // rows quad,   keys n*8 + t4*2..
-      pa[2 * n + 1] = pack2(p2, p3);  // rows quad+8
-    }
+    for (int m = 0; m < D / 16; ++m) {
+      uint32_t va[4];
+      ldsm_x4_trans(sv + sw_off<D>(wkey0 + (lane & 7) + (lane >> 4) * 8, 2 * m + ((lane >> 3) & 1)), va);
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      ps[h] += __shfl_xor_sync(0xffffffffu, ps[h], 1);
-      ps[h] += __shfl_xor_sync(0xffffffffu, ps[h], 2);
-      l_run[h] = l_run[h] * alpha[h] + ps[h];
-    }
-#pragma unroll
-    for (int n = 0; n < D / 8; ++n) {
-      oacc[n][0] *= alpha[0];
-      oacc[n][1] *= alpha[0];
-      oacc[n][2] *= alpha[1];
-      oacc[n][3] *= alpha[1];
-    }
-    // O += P V : k = this warp's 16 keys, n-tiles of 8 output dims
-#pragma unroll
-    for (int c = 0; c < C::kChunksPerRow; c += 2) {
-      uint32_t vb[4];
-      ldsm_x4_trans(sv + sw_off<D>(wkey0 + (lane & 7) + ((lane >> 3) & 1) * 8, c + (lane >> 4)), vb);
-      mma_bf16_16816(oacc[c], pa, vb[0], vb[1]);
-      mma_bf16_16816(oacc[c + 1], pa, vb[2], vb[3]);
+      for (int nt = 0; nt < kNT; ++nt) mma_bf16_16816(oacc[nt][m], va, pb[nt][0], pb[nt][1]);
     }
   }
 
-  // ---- merge the four warps through shared memory
+  // ---- merge the warps through shared memory
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1)
+#pragma unroll
+    for (int nt = 0; nt < kNT; ++nt)
+#pragma unroll
+      for (int x = 0; x < 2; ++x) l_run[nt][x] += __shfl_xor_sync(0xffffffffu, l_run[nt][x], o);
   cp_async_wait<0>();
   __syncthreads();
   constexpr int kMS = C::kMergeStride;
-  float* sc_o = reinterpret_cast<float*>(smem);               // [4][16][D + 4]
-  float* sc_ml = sc_o + 4 * 16 * kMS;                         // [4][16][2]
+  float* sc_o = reinterpret_cast<float*>(smem);               // [warps][rows][D + 4]
+  float* sc_ml = sc_o + kWarps * kRows * kMS;                 // [warps][rows][2]
 #pragma unroll
-  for (int n = 0; n < D / 8; ++n) {
-    const int d = n * 8 + t4 * 2;
-    float* r0 = sc_o + (warp * 16 + quad) * kMS + d;
-    float* r1 = sc_o + (warp * 16 + quad + 8) * kMS + d;
-    r0[0] = oacc[n][0]; r0[1] = oacc[n][1];
-    r1[0] = oacc[n][2]; r1[1] = oacc[n][3];
-  }
-  if (t4 == 0) {
-    sc_ml[(warp * 16 + quad) * 2] = m_run[0];
-    sc_ml[(warp * 16 + quad) * 2 + 1] = l_run[0];
-    sc_ml[(warp * 16 + quad + 8) * 2] = m_run[1];
-    sc_ml[(warp * 16 + quad + 8) * 2 + 1] = l_run[1];
+  for (int nt = 0; nt < kNT; ++nt) {
+    const int r = warp * kRows + nt * 8 + 2 * t4;
+#pragma unroll
+    for (int m = 0; m < D / 16; ++m) {
+      float* r0 = sc_o + r * kMS + m * 16 + quad;
+      r0[0] = oacc[nt][m][0]; r0[kMS] = oacc[nt][m][1];
+      r0[8] = oacc[nt][m][2]; r0[kMS + 8] = oacc[nt][m][3];
+    }
+    if (quad == 0) {
+      sc_ml[r * 2] = m_run[nt][0];
+      sc_ml[r * 2 + 1] = l_run[nt][0];
+      sc_ml[r * 2 + 2] = m_run[nt][1];
+      sc_ml[r * 2 + 3] = l_run[nt][1];
+    }
   }
   __syncthreads();
-  for (int idx = tid; idx < heads_here * D; idx += kThreads) {
+  float* part_o = reinterpret_cast<float*>(smem) + C::kPartOff;  // [rows][D] this CTA's unnormalised rows
+  float* part_ml = part_o + kRows * D;                           // [rows][2] (max, sum)
+  for (int idx = tid; idx < rows_here * D; idx += kThreads) {
     const int r = idx / D, d = idx % D;
     float M = -INFINITY;
 #pragma unroll
-    for (int w = 0; w < 4; ++w) M = fmaxf(M, sc_ml[(w * 16 + r) * 2]);
+    for (int w = 0; w < kWarps; ++w) M = fmaxf(M, sc_ml[(w * kRows + r) * 2]);
     float L = 0.f, acc = 0.f;
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      const float mw = sc_ml[(w * 16 + r) * 2];
+    for (int w = 0; w < kWarps; ++w) {
+      const float mw = sc_ml[(w * kRows + r) * 2];
       const float f = (mw == -INFINITY) ? 0.f : ex2f(mw - M);
-      L += sc_ml[(w * 16 + r) * 2 + 1] * f;
-      acc += sc_o[(w * 16 + r) * kMS + d] * f;
+      L += sc_ml[(w * kRows + r) * 2 + 1] * f;
+      acc += sc_o[(w * kRows + r) * kMS + d] * f;
     }
-    const int head = head0 + r;
+    if (kCluster) {
+      part_o[r * D + d] = acc;
+      if (d == 0) {
+        part_ml[2 * r] = M;
+        part_ml[2 * r + 1] = L;
+      }
+      continue;
+    }
     const float outv = acc / L;
     const float lse2 = M + log2f(L);
     if (n_chunks == 1) {
-      p.o[b * p.os[0] + (int64_t)head * p.os[1] + d] = __float2bfloat16_rn(outv);
-      if (d == 0 && p.lse) p.lse[(int64_t)b * p.n_head + head] = kLn2 * lse2;
+      o_row(p, b, hkv, row0 + r)[d] = __float2bfloat16_rn(outv);
+      if (d == 0 && p.lse) p.lse[lse_index(p, b, hkv, row0 + r)] = kLn2 * lse2;
     } else {
-      const int64_t slot = ((int64_t)b * p.n_head + head) * p.n_splits + split;
+      const int64_t slot = lse_index(p, b, hkv, row0 + r) * p.n_splits + split;
       p.ws_o[slot * D + d] = outv;
       if (d == 0) p.ws_lse[slot] = lse2;
     }
   }
+  if (kCluster) {
+    // every CTA of the cluster merges its share of the (row, dim) outputs over all CTAs' partials,
+    // eight CTAs' loads in flight at a time
+    cluster_sync();
+    const uint32_t ml0 = smem_u32(part_ml), o0 = smem_u32(part_o);
+    for (int idx = split * kThreads + tid; idx < rows_here * D; idx += p.n_splits * kThreads) {
+      const int r = idx / D, d = idx % D;
+      float M = -INFINITY, L = 0.f, acc = 0.f;
+      for (int c0 = 0; c0 < n_chunks; c0 += 8) {
+        float m8[8], l8[8], a8[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const int cc = min(c0 + c, n_chunks - 1);  // a repeated partial is given no weight below
+          const uint32_t ml = cluster_map(ml0 + 8 * r, cc);
+          m8[c] = cluster_ld_f32(ml);
+          l8[c] = cluster_ld_f32(ml + 4);
+          a8[c] = cluster_ld_f32(cluster_map(o0 + 4 * (r * D + d), cc));
+        }
+        float m_new = M;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) m_new = fmaxf(m_new, m8[c]);
+        const float f0 = ex2f(M - m_new);
+        L *= f0;
+        acc *= f0;
+        M = m_new;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const float f = c0 + c < n_chunks ? ex2f(m8[c] - M) : 0.f;
+          L = fmaf(l8[c], f, L);
+          acc = fmaf(a8[c], f, acc);
+        }
+      }
+      o_row(p, b, hkv, row0 + r)[d] = __float2bfloat16_rn(acc / L);
+      if (d == 0 && p.lse) p.lse[lse_index(p, b, hkv, row0 + r)] = kLn2 * (M + log2f(L));
+    }
+    cluster_sync();  // no CTA's shared memory goes away while another still reads it
+  }
 }
 
-// One CTA per (query head, sequence): weights w_c = 2^(L_c - max L), O = sum w_c O_c / sum w_c.
+// One CTA per (query row, sequence): weights w_c = 2^(L_c - max L), O = sum w_c O_c / sum w_c.
+// D / 4 lanes hold a row's D values, four floats each, and the CTA's 512 / D lane groups take every
+// (512 / D)-th chunk, so that the chunks' loads are in flight together: the kernel is a chain of
+// memory latencies, length, then LSEs, then partials.
 // Launched with programmatic stream serialisation: its CTAs may become resident while the split
 // kernel is still draining, and wait here until that grid has completed and its writes are visible,
 // so the launch latency of this second kernel hides behind the tail of the first.
 template <int D>
-__global__ void __launch_bounds__(D)
+__global__ void __launch_bounds__(kMergeThreads)
 decode_merge_kernel(const DecodeParams p) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  const int head = blockIdx.x, b = blockIdx.y, d = threadIdx.x;
+  constexpr int kLanes = D / 4, kGroups = kMergeThreads / kLanes;
+  __shared__ float4 s_acc[kGroups][kLanes];
+  __shared__ float s_w[kGroups];
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int row = blockIdx.x, b = blockIdx.y;  // row of the sequence: head * q_seq + query
   const int len = p.kv_lens ? min(max(p.kv_lens[b], 0), p.max_kv_seq) : p.max_kv_seq;
   const int n_chunks = (len + p.chunk_len - 1) / p.chunk_len;
   if (n_chunks <= 1) return;  // the split kernel already wrote the final row
-  const int64_t slot0 = ((int64_t)b * p.n_head + head) * p.n_splits;
-  float M = -INFINITY;
-  for (int c = 0; c < n_chunks; ++c) M = fmaxf(M, p.ws_lse[slot0 + c]);
-  float W = 0.f, acc = 0.f;
-  for (int c = 0; c < n_chunks; ++c) {
-    const float w = ex2f(p.ws_lse[slot0 + c] - M);
-    W += w;
-    acc = fmaf(w, p.ws_o[(slot0 + c) * D + d], acc);
+  const int g = threadIdx.x / kLanes, l = threadIdx.x % kLanes, lane = threadIdx.x & 31;
+  const int64_t slot0 = ((int64_t)b * p.n_head * p.q_seq + row) * p.n_splits;
+  // at most 64 chunks: every warp holds all their LSEs, two per lane
+  const float l0 = lane < n_chunks ? p.ws_lse[slot0 + lane] : -INFINITY;
+  const float l1 = lane + 32 < n_chunks ? p.ws_lse[slot0 + lane + 32] : -INFINITY;
+  float M = fmaxf(l0, l1);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+  const float w0 = ex2f(l0 - M), w1 = ex2f(l1 - M);
+  float W = 0.f;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int c0 = 0; c0 < n_chunks; c0 += kGroups) {  // warp-uniform trip count: the shuffle below needs every lane
+    const int c = c0 + g;
+    const float w = __shfl_sync(0xffffffffu, c < 32 ? w0 : w1, c & 31);
+    if (c < n_chunks) {
+      const float* vp = p.ws_o + (slot0 + c) * D + 4 * l;
+      const float4 v = p.ws_aligned ? *reinterpret_cast<const float4*>(vp) : make_float4(vp[0], vp[1], vp[2], vp[3]);
+      W += w;
+      acc.x = fmaf(w, v.x, acc.x);
+      acc.y = fmaf(w, v.y, acc.y);
+      acc.z = fmaf(w, v.z, acc.z);
+      acc.w = fmaf(w, v.w, acc.w);
+    }
   }
-  p.o[b * p.os[0] + (int64_t)head * p.os[1] + d] = __float2bfloat16_rn(acc / W);
-  if (d == 0 && p.lse) p.lse[(int64_t)b * p.n_head + head] = kLn2 * (M + log2f(W));
+  s_acc[g][l] = acc;
+  if (l == 0) s_w[g] = W;
+  __syncthreads();
+  if (g == 0) {
+#pragma unroll
+    for (int k = 1; k < kGroups; ++k) {
+      const float4 v = s_acc[k][l];
+      acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+      W += s_w[k];
+    }
+    const int head = row / p.q_seq, i = row - head * p.q_seq;
+    __nv_bfloat16* o = p.o + b * p.os[0] + (int64_t)head * p.os[1] + i * p.os[2] + 4 * l;
+    const float inv = 1.0f / W;
+    o[0] = __float2bfloat16_rn(acc.x * inv);  // element stores: the decode entries promise no alignment of O
+    o[1] = __float2bfloat16_rn(acc.y * inv);
+    o[2] = __float2bfloat16_rn(acc.z * inv);
+    o[3] = __float2bfloat16_rn(acc.w * inv);
+    if (l == 0 && p.lse) p.lse[(int64_t)b * p.n_head * p.q_seq + row] = kLn2 * (M + log2f(W));
+  }
 }
 
 // Two-way merge, natural-log LSE (the formula of RingAttn.lean:164-180).
@@ -343,48 +473,97 @@ __global__ void merge2_kernel(const float* o_a, const float* lse_a, const float*
   if (threadIdx.x == 0) lse_out[r] = L;
 }
 
-template <int D>
-int launch_d(const TyrAttnDecodeArgs& a, DecodeParams& p, cudaStream_t st) {
-  using C = DCfg<D>;
-  // per-device attribute: set on every launch so that any current device is covered
-  cudaError_t attr_err = cudaFuncSetAttribute(
-      decode_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmemBytes);
-  if (attr_err != cudaSuccess) return (int)attr_err;
-  dim3 grid(p.n_splits, a.n_kv_head * p.head_groups, a.batch);
-  decode_kernel<D><<<grid, kThreads, C::kSmemBytes, st>>>(p);
-  count_launch();
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return (int)e;
-  if (p.n_splits > 1) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(a.n_head, a.batch);
-    cfg.blockDim = dim3(D);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, decode_merge_kernel<D>, p);
-    count_launch();
-    if (e == cudaSuccess) e = cudaGetLastError();
+template <int D, int kWarps, int kNT, bool kCluster>
+cudaError_t launch_scan(const DecodeParams& p, cudaStream_t st) {
+  constexpr int kSmem = DCfg<D, kWarps, kNT>::kSmemBytes;
+  static std::atomic<bool> attr_set[64] = {};  // per device
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  if (!attr_set[dev].load(std::memory_order_acquire)) {
+    e = cudaFuncSetAttribute(decode_kernel<D, kWarps, kNT, kCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    if (e == cudaSuccess && kCluster)
+      e = cudaFuncSetAttribute(decode_kernel<D, kWarps, kNT, kCluster>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    attr_set[dev].store(true, std::memory_order_release);
   }
-  return (int)e;
+  return launch_overlapped(decode_kernel<D, kWarps, kNT, kCluster>, dim3(p.n_splits, p.n_kv_head * p.row_groups, p.batch), dim3(32 * kWarps),
+                           kSmem, st, kCluster ? p.n_splits : 1, p);
 }
+
+// How a launch cuts its keys.
+struct ScanPlan {
+  bool cluster;   // n_splits CTAs per (sequence, KV head, row group) merge among themselves; else chunk_len keys per CTA
+  int n_splits, chunk_len, warps;
+};
+
+template <int D, int kNT>
+cudaError_t launch_scan_of(const DecodeParams& p, const ScanPlan& s, cudaStream_t st) {
+  if (s.cluster) return s.warps == 8 ? launch_scan<D, 8, kNT, true>(p, st) : launch_scan<D, 4, kNT, true>(p, st);
+  return s.warps == 8 ? launch_scan<D, 8, kNT, false>(p, st) : launch_scan<D, 4, kNT, false>(p, st);
+}
+
+template <int D>
+int launch_d(DecodeParams& p, const ScanPlan& s, cudaStream_t st) {
+  p.n_splits = s.n_splits;
+  p.chunk_len = s.chunk_len;
+  cudaError_t e = p.rows <= 8 ? launch_scan_of<D, 1>(p, s, st) : launch_scan_of<D, 2>(p, s, st);
+  count_launch();
+  if (e != cudaSuccess) return (int)e;
+  if (!s.cluster && p.n_splits > 1) {
+    e = launch_overlapped(decode_merge_kernel<D>, dim3(p.n_head * p.q_seq, p.batch), dim3(kMergeThreads), 0, st, 1, p);
+    count_launch();
+  }
+  return (int)(e != cudaSuccess ? e : cudaGetLastError());
+}
+
+constexpr int kChunkUnit = 64;  // keys; chunk lengths are multiples of it
+
+// The cut of a launch small enough to be done without a workspace: one chunk per (sequence, KV head), or a
+// cluster of CTAs for each.  `units`: (sequence, KV head, row group) triples.  Returns false for launches
+// that a cut into chunks of the workspace form serves better.
+//
+// The most CTAs that still run all at once, clusters placed: two per SM less the slots a GPC cannot
+// give to whole clusters.  Clusters of 16 leave more of them unused and are only taken where half the
+// slots are enough (for head_dim 64 three quarters).  A CTA gets at least one step of its warps' keys (64 or 128); past
+// 1024 (head_dim 64: 2048) keys per CTA the workspace form's greater choice of chunk counts wins.
+// Device time, workspace form -> this one, 8 KV heads of 128: one sequence of 512 keys 8.2 -> 4.8 us,
+// 1537: 8.8 -> 6.7, 4096: 9.5 -> 8.5, 16384: 18.9 -> 18.3 (32768: 29.2 -> 30.7, not taken); 4 x 2051 12.6 -> 10.8,
+// 4 x 8192 27.1 -> 24.2; 8 x 1537 14.2 -> 13.2; 12 KV heads of 64: 1537 7.1 -> 5.4, 4 x 8192 23.7 -> 20.0.
+// Eight warps per CTA instead of four where one CTA has an SM to itself, and for head_dim 64, whose
+// stages are half as large.
+bool small_scan_plan(int head_dim, long long units, int max_len, int max_splits, ScanPlan* s) {
+  const int sm = sm_count(), slots = 2 * sm - sm / 4;
+  const int warps = head_dim == 64 ? 8 : 4;
+  int n = (int)std::min<long long>(8, slots / std::max<long long>(units, 1));
+  if (units * 16 <= (head_dim == 64 ? slots * 3 / 4 : slots / 2)) n = 16;
+  n = std::min(n, (max_len + kWarpKeys * warps - 1) / (kWarpKeys * warps));
+  n = std::max(std::min(n, max_splits), 1);
+  if (max_len > (head_dim == 64 ? 2048 : 1024) * n) return false;
+  // few, long pieces that leave a quarter of the slots empty (4 x 24 KV heads, 2000 keys: 29.2 against 25.7 us)
+  if (n > 1 && n < 8 && max_len > 512 * n && units * n * 4 < slots * 3) return false;
+  s->cluster = n > 1;
+  s->n_splits = n;
+  s->chunk_len = n > 1 ? 0 : (max_len + kChunkUnit - 1) / kChunkUnit * kChunkUnit;
+  s->warps = n > 1 ? warps : (units <= sm ? 8 : 4);
+  return true;
+}
+
+int max_splits_of(int max_splits) { return max_splits <= 0 || max_splits > 64 ? 64 : max_splits; }
 
 }  // namespace
 
 int decode_num_splits(int max_kv_seq, int max_splits, int* chunk_len) {
-  if (max_splits <= 0 || max_splits > 64) max_splits = 64;
+  max_splits = max_splits_of(max_splits);
   int chunk = (max_kv_seq + max_splits - 1) / max_splits;
-  chunk = (chunk + kTileKeys - 1) / kTileKeys * kTileKeys;
+  chunk = (chunk + kChunkUnit - 1) / kChunkUnit * kChunkUnit;
   if (chunk < kMinChunk) chunk = kMinChunk;
   if (chunk_len) *chunk_len = chunk;
   return (max_kv_seq + chunk - 1) / chunk;
 }
 
-// Chunk length of a launch.  decode_num_splits gives the most chunks the workspace is sized for;
+// Chunk length of a launch that goes through the workspace.  decode_num_splits gives the most chunks the workspace is sized for;
 // a launch uses longer chunks than that when it can: every CTA pays for filling its load pipeline,
 // the cross-warp merge and a partial output row.
 //  * A launch with at least four CTAs for every CTA slot of the device at 2048-key chunks takes
@@ -409,16 +588,16 @@ int decode_launch_splits(int max_kv_seq, int max_splits, int batch, int ctas_per
     if (total_kv_len > 0) return ctas_per_seq_chunk * (total_kv_len / chunk + (batch + 1) / 2);
     return (long long)ctas_per_seq_chunk * batch * ((max_kv_seq + chunk - 1) / chunk);
   };
-  const int whole = (max_kv_seq + kTileKeys - 1) / kTileKeys * kTileKeys;  // one chunk per sequence
+  const int whole = (max_kv_seq + kChunkUnit - 1) / kChunkUnit * kChunkUnit;  // one chunk per sequence
   int chunk = 2048;
   if (ctas(chunk) < 4 * slots) {
     long long one_wave = 0;  // chunk length of the one-wave cut, 0 when the launch does not take it
     if (lengths_known && ctas(chunk) < 3 * slots) {
       const long long keys = total_kv_len > 0 ? total_kv_len : (long long)batch * max_kv_seq;
       long long c = (keys * ctas_per_seq_chunk + slots - 1) / slots;
-      c = (c + kTileKeys - 1) / kTileKeys * kTileKeys;
+      c = (c + kChunkUnit - 1) / kChunkUnit * kChunkUnit;
       c = std::min<long long>(std::max<long long>(c, kMinChunk), whole);
-      while (c < whole && ctas((int)c) > slots) c += kTileKeys;
+      while (c < whole && ctas((int)c) > slots) c += kChunkUnit;
       // short sequences, many of them: even one CTA per (sequence, KV head) is more than a wave
       if (ctas((int)c) <= slots) one_wave = c;
     }
@@ -451,16 +630,16 @@ int launch_decode(const TyrAttnDecodeArgs& a, float scale, cudaStream_t st) {
   p.kv_lens = a.kv_lens;
   p.kv_head_strides = a.kv_head_strides;
   p.batch = a.batch; p.n_head = a.n_head; p.n_kv_head = a.n_kv_head; p.max_kv_seq = a.max_kv_seq;
-  p.group = a.n_head / a.n_kv_head;
-  p.head_groups = (p.group + 15) / 16;
+  p.q_seq = 1;
+  p.rows = a.n_head / a.n_kv_head;
+  p.row_groups = (p.rows + 15) / 16;
   for (int i = 0; i < 2; ++i) { p.qs[i] = a.q_stride[i]; p.os[i] = a.o_stride[i]; }
+  p.qs[2] = p.os[2] = 0;
   for (int i = 0; i < 3; ++i) { p.ks[i] = a.k_stride[i]; p.vs[i] = a.v_stride[i]; }
   p.scale_log2 = scale * kLog2e;
-  p.n_splits = decode_launch_splits(a.max_kv_seq, a.max_splits, a.batch, a.n_kv_head * p.head_groups,
-                                    a.total_kv_len > 0 ? a.total_kv_len : 0, a.kv_lens == nullptr || a.total_kv_len > 0,
-                                    &p.chunk_len);
   p.ws_o = nullptr;
   p.ws_lse = nullptr;
+  p.ws_aligned = 1;
   {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return -TYR_ATTN_ERR_NO_DEVICE;
@@ -468,15 +647,84 @@ int launch_decode(const TyrAttnDecodeArgs& a, float scale, cudaStream_t st) {
     if (!ds) return -TYR_ATTN_ERR_NO_DEVICE;
     p.status = ds->status;
   }
-  if (p.n_splits > 1) {
+  ScanPlan s{false, 1, 0, 4};
+  s.n_splits = decode_launch_splits(a.max_kv_seq, a.max_splits, a.batch, a.n_kv_head * p.row_groups,
+                                    a.total_kv_len > 0 ? a.total_kv_len : 0, a.kv_lens == nullptr || a.total_kv_len > 0,
+                                    &s.chunk_len);
+  if (s.n_splits > 1) {  // the workspace is asked for whether or not this launch then uses it
     const size_t need = decode_workspace_bytes(a.batch, a.n_head, a.head_dim, a.max_kv_seq, a.max_splits);
     if (a.workspace == nullptr || a.workspace_bytes < need) return -TYR_ATTN_ERR_WORKSPACE;
     p.ws_o = static_cast<float*>(a.workspace);
-    p.ws_lse = p.ws_o + (size_t)a.batch * a.n_head * p.n_splits * a.head_dim;
+    p.ws_lse = p.ws_o + (size_t)a.batch * a.n_head * s.n_splits * a.head_dim;
+    p.ws_aligned = (reinterpret_cast<uintptr_t>(p.ws_o) & 15) == 0;
   }
-  if (a.head_dim == 128) return launch_d<128>(a, p, st);
-  if (a.head_dim == 64) return launch_d<64>(a, p, st);
+  small_scan_plan(a.head_dim, (long long)a.batch * a.n_kv_head * p.row_groups, a.max_kv_seq, max_splits_of(a.max_splits), &s);
+  if (a.head_dim == 128) return launch_d<128>(p, s, st);
+  if (a.head_dim == 64) return launch_d<64>(p, s, st);
   return -TYR_ATTN_ERR_HEAD_DIM;
+}
+
+// ---- the typed call with few query rows per KV head
+namespace {
+
+ScanPlan few_rows_plan(const TyrAttnPrefillArgs& a, bool have_workspace) {
+  const int rows = a.n_head / a.n_kv_head * a.q_seq;
+  const long long units = (long long)a.batch * a.n_kv_head * ((rows + 15) / 16);
+  ScanPlan s{false, 1, 0, 4};
+  const bool small = small_scan_plan(a.head_dim, units, a.kv_seq, 64, &s);
+  // One or two (batch, KV head) pairs over at least 1024 keys keep to the workspace where the caller gives
+  // one, as such calls always have: it reaches more of the device than two clusters of 16 can (one
+  // sequence of 16384 keys, two KV heads: 12.5 us against 13.2; of 1500 keys 6.8 against 4.7).
+  if (!have_workspace || (small && !(units <= 2 && a.kv_seq >= 1024))) return s;
+  // chunks that give one wave of CTAs, as in decode_launch_splits
+  const int slots = 2 * sm_count();
+  long long c = ((long long)a.kv_seq * units + slots - 1) / slots;
+  c = std::max<long long>(c, (a.kv_seq + 63) / 64);
+  s.cluster = false;
+  s.warps = 4;
+  s.chunk_len = (int)((c + kChunkUnit - 1) / kChunkUnit * kChunkUnit);
+  s.n_splits = (a.kv_seq + s.chunk_len - 1) / s.chunk_len;
+  return s;
+}
+
+}  // namespace
+
+bool few_rows_call(const TyrAttnPrefillArgs& a) {
+  return !a.is_causal && a.window_size == 0 && a.key_mask == nullptr && !a.check_mode && a.dtype == TYR_ATTN_BF16 &&
+         (a.head_dim == 64 || a.head_dim == 128) && (long long)a.n_head / a.n_kv_head * a.q_seq <= kMaxFewRows;
+}
+
+size_t few_rows_workspace_bytes(const TyrAttnPrefillArgs& a) {
+  const ScanPlan s = few_rows_plan(a, true);
+  if (s.cluster || s.n_splits <= 1) return 0;
+  return (size_t)a.batch * a.n_head * a.q_seq * s.n_splits * ((size_t)a.head_dim + 1) * sizeof(float);
+}
+
+int launch_few_rows(const TyrAttnPrefillArgs& a, float scale, int* status, cudaStream_t st) {
+  DecodeParams p;
+  p.q = static_cast<const __nv_bfloat16*>(a.q);
+  p.o = static_cast<__nv_bfloat16*>(a.o);
+  p.lse = a.lse;
+  p.k = static_cast<const __nv_bfloat16*>(a.k);
+  p.v = static_cast<const __nv_bfloat16*>(a.v);
+  p.k_ptrs = p.v_ptrs = nullptr;
+  p.kv_lens = nullptr;
+  p.kv_head_strides = nullptr;
+  p.batch = a.batch; p.n_head = a.n_head; p.n_kv_head = a.n_kv_head; p.max_kv_seq = a.kv_seq;
+  p.q_seq = a.q_seq;
+  p.rows = a.n_head / a.n_kv_head * a.q_seq;
+  p.row_groups = (p.rows + 15) / 16;
+  for (int i = 0; i < 3; ++i) { p.qs[i] = a.q_stride[i]; p.os[i] = a.o_stride[i]; p.ks[i] = a.k_stride[i]; p.vs[i] = a.v_stride[i]; }
+  p.scale_log2 = scale * kLog2e;
+  p.status = status;
+  const size_t need = few_rows_workspace_bytes(a);
+  const bool ws = a.workspace != nullptr && need > 0 && (size_t)a.workspace_bytes >= need &&
+                  (reinterpret_cast<uintptr_t>(a.workspace) & 255) == 0;
+  const ScanPlan s = few_rows_plan(a, ws);
+  p.ws_o = static_cast<float*>(a.workspace);
+  p.ws_lse = ws ? p.ws_o + (size_t)a.batch * a.n_head * a.q_seq * s.n_splits * a.head_dim : nullptr;
+  p.ws_aligned = 1;
+  return a.head_dim == 128 ? launch_d<128>(p, s, st) : launch_d<64>(p, s, st);
 }
 
 int launch_merge2(const float* o_a, const float* lse_a, const float* o_b, const float* lse_b,

@@ -1,6 +1,5 @@
-// Warp-level building blocks of the two latency-bound kernels (single-token decode, short-sequence
-// prefill): 16-byte cp.async, ldmatrix and the m16n8k16 bf16 MMA.  These kernels spend their time
-// waiting for memory or for a short dependency chain, not in the tensor pipe, so they use many
+// Warp-level building blocks of the decode kernel: 16-byte cp.async, ldmatrix and the m16n8k16 bf16
+// MMA.  It waits for memory or for a short dependency chain, not for the tensor pipe, so it uses many
 // small CTAs per SM instead of the one-CTA-per-SM tcgen05 pipeline.
 #pragma once
 #include <cuda_bf16.h>
@@ -33,6 +32,12 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], const uint32_t (&a
       "{%8, %9}, {%0, %1, %2, %3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// lane (row r, column pair c) of an 8 x 8 block of 16-bit values gets (row c.., column r): the block transposed
+__device__ __forceinline__ uint32_t transpose_8x8(uint32_t x) {
+  uint32_t y;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+  return y;
 }
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   uint32_t r;
