@@ -139,7 +139,7 @@ struct Cfg {
   static constexpr bool kStageO = (D == 128);
   static constexpr uint32_t kOOff = kVOff + kVStages * kTileBytes;  // one O tile staged for its TMA store
   static constexpr uint32_t kBarOff = kOOff + kTileBytes;
-  static constexpr int kNumBars = 2 + 2 + 2 * kKStages + 2 * kVStages + 2 + 2 + 2 + 2 + 1 + 2;
+  static constexpr int kNumBars = 2 + 2 + 2 * kKStages + 2 * kVStages + 2 + 2 + 2 + 2 + 1 + 2 + 4;
   static constexpr uint32_t kSmemBytes = kBarOff + kNumBars * 8 + 16 + 1024;  // + align slack
   static constexpr uint32_t kTmemCols = 512;
   static constexpr uint32_t kTmemS = 0, kTmemO = 256;
@@ -163,7 +163,10 @@ struct Bars {
   static constexpr int o_full = p_full + 2;               // [2] last PV_t of the item done
   static constexpr int o_staged = o_full + 2;             // an O tile is in the staging buffer (4 warp arrivals)
   static constexpr int o_stage_free = o_staged + 1;       // [2] the TMA store of Q tile t's O has read the buffer
+  static constexpr int rng_full = o_stage_free + 2;       // [2] padding mask: the item's range of KV tiles is known
+  static constexpr int rng_empty = rng_full + 2;          // [2] every role has read it (producer, issuer, 8 softmax warps)
   __device__ static constexpr uint32_t count(int i) {
+    if (i >= rng_empty) return 10u;
     return ((i >= p_half && i < p_half + 4) || i == o_staged) ? 4u : 1u;  // one arrival per softmax warp
   }
 };
@@ -181,6 +184,9 @@ struct Item {
   int n0, n1;  // KV tiles Q tile 0 / Q tile 1 visit, counted from `lo`
   int part_slot;  // -1, or (part of the keys this work item covers) * n_split + index among the split items
 };
+// Masks compiled into a kernel beyond the causal one: none, the sliding window, or the padding mask (with
+// or without a window).
+constexpr int kNoMask = 0, kWindowMask = 1, kKeyMask = 2;
 // Two ways to fill the two Q-tile slots of an item:
 //  rows  : 256 consecutive rows of one query head (tile 1 sits 128 rows below tile 0);
 //  heads : the same 128 rows of two query heads that share a KV head (GQA).  Both tiles
@@ -191,7 +197,7 @@ struct Item {
 // the decode sat on the path between them: 24.4 -> 22.7 us).  With the long items of the D=128
 // workloads nothing is gained at the boundary, and that form of this function measured 3 % slower
 // there (1113 vs 1154 TFLOP/s, either order), so they keep the plain divisions.
-template <bool kWindow, bool kFast>
+template <int kMask, bool kFast>
 __device__ __forceinline__ Item decode_item(int w, const PrefillParams& p) {
   Item it;
   const int n_groups = p.batch * p.n_kv_head;
@@ -242,7 +248,7 @@ __device__ __forceinline__ Item decode_item(int w, const PrefillParams& p) {
   // Sliding window: the first row of the item sees no key before row - window + 1.  Both
   // Q tiles start at that tile; a tile that lies wholly before a row's window is masked
   // out for that row (the softmax copes with rows that have seen no key yet).
-  it.lo = (kWindow && p.window > 0) ? max(0, it.row[0] - p.window + 1) / kBN : 0;
+  it.lo = (kMask != kNoMask && p.window > 0) ? max(0, it.row[0] - p.window + 1) / kBN : 0;
   it.n0 = (p.causal ? min(nkv_total, last0) : nkv_total) - it.lo;
   it.n1 = (p.causal ? min(nkv_total, last1) : nkv_total) - it.lo;
   return it;
@@ -270,22 +276,62 @@ __device__ __forceinline__ int item_of_table(int it, const PrefillParams& p) {
 
 // Work item w of the launch: the items before p.split_from as they are, the ones from there on as
 // two to eight parts of their KV tiles each (non-causal launches only, so both Q tiles visit every tile).
-template <int D, bool kWindow, bool kSplit>
+template <int D, int kMask, bool kSplit>
 __device__ __forceinline__ Item work_item(int w, const PrefillParams& p) {
   if (!kSplit || w < p.split_from) {
-    Item it = decode_item<kWindow, D == 64>(w, p);
+    Item it = decode_item<kMask, D == 64>(w, p);
     it.part_slot = -1;
     return it;
   }
   const int s = w - p.split_from;
   const int slot = p.by_parts.div(s);
   const int part = s - slot * p.n_parts;
-  Item it = decode_item<kWindow, D == 64>(p.split_from + slot, p);
+  Item it = decode_item<kMask, D == 64>(p.split_from + slot, p);
   const int n = it.n1;  // KV tiles of the whole item; part k covers tiles [k n / parts, (k + 1) n / parts)
   it.part_slot = part * p.n_split + slot;
   it.lo = part * n / p.n_parts;
   it.n0 = it.n1 = (part + 1) * n / p.n_parts - it.lo;
   return it;
+}
+
+// Padding masks: KV tiles in front of the first and behind the last tile with a valid key are not visited.
+// Returns the item's (lo, n0, n1) cut down to those between them; each Q tile keeps at least one KV tile (a
+// batch row without a valid key in reach: its rows come out as NaN, as from ATen).  Looks at four tiles at a
+// time from either end, so a batch row padded on one side takes a round or two per end.
+// Not inlined: its registers would be the kernel's (scores of a whole row are live elsewhere).
+// The masked launches are bound like the others by softmax and tensor pipe, so a tile not visited is time saved,
+// and the look-up runs on an idle warp two items ahead.  With the mask bytes fetched before the wait for the
+// scores: 8 causal prompts of up to 1111 rows 75.2 -> 64.8 us, 4 x 2000 rows x 24 heads, not causal, 264 -> 174 us.
+__device__ __noinline__ int4 valid_tiles(const uint8_t* mrow, int kv_seq, int lo, int n0, int n1) {
+  const int lane = threadIdx.x & 31;
+  const int end = lo + n1, end0 = lo + n0;
+  auto any4 = [&](int j0) {  // bit x: tile j0 + x is in [lo, end) and has a valid key
+    uint32_t any = 0;
+    uint32_t v[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int kk = (j0 + x) * kBN + c * 32 + lane;
+        if (j0 + x >= lo && j0 + x < end && kk < kv_seq) v[x] |= __ldg(mrow + kk);
+      }
+#pragma unroll
+    for (int x = 0; x < 4; ++x) any |= (__any_sync(0xffffffffu, v[x] != 0u) ? 1u : 0u) << x;
+    return any;
+  };
+  int first = lo, last = -1;
+  for (int j0 = end - 4; last < 0 && j0 + 3 >= lo; j0 -= 4) {
+    const uint32_t any = any4(j0);
+    if (any) last = j0 + 31 - __clz(any);
+  }
+  if (last < 0) return make_int4(lo, 1, 1, 0);
+  for (uint32_t any = 0; any == 0; first += 4) {  // ends at tile `last` at the latest
+    any = any4(first);
+    if (any) first += __ffs(any) - 1 - 4;
+  }
+  first = min(first, end0 - 1);
+  n0 = max(1, min(end0, last + 1) - first);
+  return make_int4(first, n0, max(n0, last + 1 - first), 0);
 }
 
 // The issuing thread shares its SM sub-partition with two softmax warps, so every
@@ -372,10 +418,10 @@ __device__ __forceinline__ void exp_chunk(const uint32_t (&sr)[32], uint64_t sl2
 // run on across items (every role counts its own uses), tensor memory and the
 // barriers are set up once, the next item's Q/K loads and first QK^T overlap the
 // previous item's epilogue.
-// kWindow compiles the sliding-window and padding-key masks in (rows may then meet tiles in
-// which they see no key); the plain kernel carries none of those checks.
+// kMask compiles the sliding window or the padding mask in (rows may then meet tiles in which they see no
+// key); the plain kernel carries none of those checks.
 // kSplit compiles the key-split of the last round in (work_item); the plain kernel has no trace of it.
-template <int D, bool kWindow, bool kSplit, bool kTabled>
+template <int D, int kMask, bool kSplit, bool kTabled>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
@@ -385,6 +431,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint32_t tmem_slot;
   __shared__ WaitCtl wait_ctl;
+  __shared__ int4 key_range[kMask == kKeyMask ? 2 : 1];  // (lo, n0, n1) of this CTA's items in flight (kKeyMask)
 
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;  // 128B-swizzle atoms need 1024-byte alignment
@@ -417,6 +464,22 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   const uint32_t tmem = tmem_slot;
   volatile WaitCtl* abortp = &wait_ctl;
 
+  // Padding mask: cuts item number `it` of this CTA down to the tiles with a valid key, which the scan warp
+  // has looked up.  Called once per item by the producing lane and by the issuing and softmax warps.
+  auto cut_to_keys = [&](Item& im, int it, bool whole_warp) {
+    if (kMask != kKeyMask) return true;
+    bool got = mbar_wait(bar(B::rng_full + (it & 1)), (it >> 1) & 1, abortp);
+    if (whole_warp) got = __all_sync(0xffffffffu, got);
+    if (!got) return false;
+    const int4 cut = key_range[it & 1];
+    im.lo = cut.x;
+    im.n0 = cut.y;
+    im.n1 = cut.z;
+    if (whole_warp) __syncwarp();
+    if (!whole_warp || lane == 0) mbar_arrive(bar(B::rng_empty + (it & 1)));
+    return true;
+  };
+
   // Register budget: the four warps of the first warpgroup only issue copies and
   // MMAs; the softmax warpgroups hold a whole 128-column score row per thread.
   if (warp < 4) {
@@ -429,7 +492,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         for (int it = 0; ok; ++it) {
           const int w = kTabled ? item_of_table(it, p) : snake_item(it, total_items, p.snake);
           if (w < 0) break;
-          const Item im = work_item<D, kWindow, kSplit>(w, p);
+          Item im = work_item<D, kMask, kSplit>(w, p);
 #pragma unroll
           for (int t = 0; t < 2; ++t) {
             if (it > 0) ok = ok && mbar_wait(bar(B::q_empty + t), (it - 1) & 1, abortp);
@@ -462,6 +525,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                           (im.lo + j) * kBN, im.hkv, im.b);
             ++vc;
           };
+          if (ok) ok = cut_to_keys(im, it, false);
           if (ok) load_k(0);
           for (int j = 0; j < im.n1 && ok; ++j) {
             if (j + 1 < im.n1) load_k(j + 1);
@@ -484,7 +548,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         for (int it = 0; ok; ++it) {
           const int w = kTabled ? item_of_table(it, p) : snake_item(it, total_items, p.snake);
           if (w < 0) break;
-          const Item im = work_item<D, kWindow, kSplit>(w, p);
+          Item im = work_item<D, kMask, kSplit>(w, p);
+          if (!cut_to_keys(im, it, true)) break;
           const int n0 = im.n0, n1 = im.n1;
           ok = mbar_wait(bar(B::q_full + 0), it & 1, abortp) && mbar_wait(bar(B::q_full + 1), it & 1, abortp) &&
                mbar_wait(bar(B::k_full + kc % C::kKStages), (kc / C::kKStages) & 1, abortp);
@@ -562,6 +627,23 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           }
         }
       }
+    } else if (warp == 2 && kMask == kKeyMask) {
+      // -------------------------------------------------------- scan
+      // Looks up the range of KV tiles with a valid key, up to two items ahead of the other roles.
+      bool ok = true;
+      for (int it = 0; ok; ++it) {
+        const int w = kTabled ? item_of_table(it, p) : snake_item(it, total_items, p.snake);
+        if (w < 0) break;
+        const Item im = work_item<D, kMask, kSplit>(w, p);
+        const int4 cut = valid_tiles(p.key_mask + im.b * p.key_mask_stride, p.kv_seq, im.lo, im.n0, im.n1);
+        if (it >= 2) ok = __all_sync(0xffffffffu, mbar_wait(bar(B::rng_empty + (it & 1)), ((it >> 1) - 1) & 1, abortp));
+        if (!ok) break;
+        if (lane == 0) {
+          key_range[it & 1] = cut;
+          mbar_arrive(bar(B::rng_full + (it & 1)));
+        }
+        __syncwarp();
+      }
     } else if (warp == 3) {
       // -------------------------------------------------------- O store
       // The softmax warps put a finished O tile into the staging buffer as bf16 (row-per-thread
@@ -575,7 +657,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         for (int it = 0; ok; ++it) {
           const int w = kTabled ? item_of_table(it, p) : snake_item(it, total_items, p.snake);
           if (w < 0) break;
-          const Item im = work_item<D, kWindow, kSplit>(w, p);
+          const Item im = work_item<D, kMask, kSplit>(w, p);
 #pragma unroll
           for (int t = 0; t < 2; ++t, ++u) {
             ok = mbar_wait(bar(B::o_staged), u & 1, abortp);
@@ -610,19 +692,36 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     const uint32_t tS = tmem + lane_addr + C::kTmemS + t * kBN;
     const uint32_t tO = tmem + lane_addr + C::kTmemO + t * D;
     const float sl2 = p.scale_log2;
+    constexpr bool kRefByRow = kMask != kNoMask;  // rows may meet tiles in which they see no key
     bool ok = true;
     int sc = 0;  // score tiles of this Q-tile slot processed so far, over all items
 
     for (int it = 0; ok; ++it) {
       const int w = kTabled ? item_of_table(it, p) : snake_item(it, total_items, p.snake);
       if (w < 0) break;
-      const Item im = work_item<D, kWindow, kSplit>(w, p);
+      Item im = work_item<D, kMask, kSplit>(w, p);
+      if (!cut_to_keys(im, it, true)) break;
       const int row = (t ? im.row[1] : im.row[0]) + r;  // query index
       const int hq = t ? im.hq[1] : im.hq[0];
+      // the KV tiles by their first key (kRefByRow) or by number: the former keeps registers free where the
+      // range comes from memory, the latter measured 4 % faster in the plain instantiation at D = 64
       const int n_t = t ? im.n1 : im.n0;
+      const int j_begin = kRefByRow ? im.lo * kBN : 0, j_end = kRefByRow ? (im.lo + n_t) * kBN : n_t;
+      const int j_step = kRefByRow ? kBN : 1;
       float m_ref = -INFINITY, l = 0.f;
 
-      for (int j = 0; j < n_t; ++j, ++sc) {
+      for (int j = j_begin; j < j_end; j += j_step, ++sc) {
+        const int key0 = kRefByRow ? j : (im.lo + j) * kBN;  // first key of the tile
+        // padding keys: lane i fetches the mask bytes of keys i, 32 + i, 64 + i, 96 + i of the tile, before
+        // the wait for the scores, where the warp has time
+        uint32_t valid4 = 0;
+        if (kMask == kKeyMask) {
+          const int kk = key0 + lane;
+          const uint8_t* mrow = p.key_mask + im.b * p.key_mask_stride + kk;
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            if (kk + 32 * c < p.kv_seq && __ldg(mrow + 32 * c) != 0) valid4 |= 1u << c;
+        }
         ok = mbar_wait(bar(B::s_full + t), sc & 1, abortp);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
@@ -635,29 +734,23 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         for (int c = 0; c < kBN / 32; ++c) tmem_ld_ready(sr[c]);
 
         // keys this row may see in this tile: [first, limit)
-        const int key0 = (im.lo + j) * kBN;
         int limit = p.kv_seq - key0;
         if (p.causal) limit = min(limit, row + 1 - key0);
-        const int first = (kWindow && p.window > 0) ? row - p.window + 1 - key0 : 0;
+        const int first = (kMask != kNoMask && p.window > 0) ? row - p.window + 1 - key0 : 0;
         if (limit < kBN || first > 0) {
 #pragma unroll
           for (int c = 0; c < kBN; ++c)
             if (c >= limit || c < first) sr[c >> 5][c & 31] = 0xff800000u;  // -inf
         }
-        if (kWindow && p.key_mask != nullptr) {
-          // padding keys: lane i fetches the mask bytes of keys 4i..4i+3 of the tile, four
-          // ballots spread them to every row; key c is bit (c >> 2) of ballot (c & 3)
-          const uint8_t* mrow = p.key_mask + im.b * p.key_mask_stride + key0;
-          uint32_t vb[4];
+        if (kMask == kKeyMask && __any_sync(0xffffffffu, valid4 != 0xfu)) {
+          // a ballot per 32 keys spreads the bytes to every row
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int kk = 4 * lane + e;
-            const bool valid = (key0 + kk < p.kv_seq) && mrow[kk] != 0;
-            vb[e] = __ballot_sync(0xffffffffu, valid);
+          for (int c = 0; c < 4; ++c) {
+            const uint32_t valid = __ballot_sync(0xffffffffu, (valid4 >> c) & 1u);
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (!((valid >> i) & 1u)) sr[c][i] = 0xff800000u;  // -inf
           }
-#pragma unroll
-          for (int c = 0; c < kBN; ++c)
-            if (!((vb[c & 3] >> (c >> 2)) & 1u)) sr[c >> 5][c & 31] = 0xff800000u;  // -inf
         }
         float mxa[4];
 #pragma unroll
@@ -673,15 +766,17 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         const float mx = fmaxf(fmaxf(mxa[0], mxa[1]), fmaxf(mxa[2], mxa[3]));
 
         const float m_new = fmaxf(m_ref, mx);
-        if (j == 0) {
+        // a row that has seen no key yet has l = 0 and nothing but zeros in O_t, or no O_t yet
+        if (kRefByRow && m_ref == -INFINITY) m_ref = m_new;
+        if (!kRefByRow && j == 0) {
           m_ref = m_new;
         } else {
           const bool grow = (m_new - m_ref) * sl2 > kRescaleThreshold;
           if (__any_sync(0xffffffffu, grow)) {
             // PV_t(j-1) has completed (s_full covers it) and PV_t(j) is not issued
             // before this warp arrives on p_half, so O_t is ours to rescale.
-            // a row that has seen no key yet (m_new still -inf, sliding window only) keeps its zeros
-            const float alpha = (kWindow && m_new == -INFINITY) ? 1.0f : ex2_approx((m_ref - m_new) * sl2);
+            // (-inf - -inf: a row that has still seen no key)
+            const float alpha = (kRefByRow && m_new == -INFINITY) ? 1.0f : ex2_approx((m_ref - m_new) * sl2);
             l *= alpha;
             m_ref = m_new;
 #pragma unroll
@@ -696,13 +791,13 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             }
           }
         }
-        const float neg = (kWindow && m_ref == -INFINITY) ? 0.0f : -m_ref * sl2;  // all -inf scores give P = 0
+        const float neg = (kRefByRow && m_ref == -INFINITY) ? 0.0f : -m_ref * sl2;  // all -inf scores give P = 0
         const uint64_t sl2x2 = pack_f32x2(sl2, sl2), negx2 = pack_f32x2(neg, neg);
         uint64_t sum_a = pack_f32x2(0.f, 0.f), sum_b = sum_a;
 #pragma unroll
         for (int c = 0; c < kBN / 32; ++c) {
           uint32_t pk[16];
-          exp_chunk<kWindow ? 0 : kExpPolyPairs>(sr[c], sl2x2, negx2, pk, sum_a, sum_b);
+          exp_chunk<kMask != kNoMask ? 0 : kExpPolyPairs>(sr[c], sl2x2, negx2, pk, sum_a, sum_b);
           tmem_st16(tS + c * 16, pk);
           if (c == 1) {  // keys 0..63 of P are in tensor memory: the first half of PV may start
             tmem_wait_st();
@@ -926,7 +1021,7 @@ __global__ void __launch_bounds__(256) prefill_split_merge_kernel(const PrefillP
   const int col = (lane % kLanesPerRow) * 8;
   const int r = id & (kBM - 1), t = (id >> 7) & 1, slot = id >> 8;
   if (slot >= p.n_split) return;
-  const Item im = decode_item<false, true>(p.split_from + slot, p);
+  const Item im = decode_item<kNoMask, true>(p.split_from + slot, p);
   const int row = im.row[t] + r;
   if (row >= p.q_seq) return;
   const int hq = im.hq[t];
@@ -1033,7 +1128,7 @@ bool item_table_for(PrefillParams& p, int grid, cudaStream_t st) {
   return true;
 }
 
-template <int D, bool kWindow>
+template <int D, int kMask>
 int launch(const TyrAttnPrefillArgs& a, float scale, int* status, cudaStream_t st) {
   using C = Cfg<D>;
   CUtensorMap tq, tk, tv, to;
@@ -1048,17 +1143,17 @@ int launch(const TyrAttnPrefillArgs& a, float scale, int* status, cudaStream_t s
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -TYR_ATTN_ERR_NO_DEVICE;
     if (!attr_set[dev].load(std::memory_order_acquire)) {
-      cudaError_t attr_err = cudaFuncSetAttribute(prefill_kernel<D, kWindow, false, false>,
+      cudaError_t attr_err = cudaFuncSetAttribute(prefill_kernel<D, kMask, false, false>,
                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   (int)C::kSmemBytes);
       if (attr_err != cudaSuccess) return (int)attr_err;
-      if (!kWindow) {
-        attr_err = cudaFuncSetAttribute(prefill_kernel<D, false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      if (kMask == kNoMask) {
+        attr_err = cudaFuncSetAttribute(prefill_kernel<D, kNoMask, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)C::kSmemBytes);
         if (attr_err != cudaSuccess) return (int)attr_err;
       }
-      if (!kWindow && D == 128) {
-        attr_err = cudaFuncSetAttribute(prefill_kernel<128, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      if (kMask == kNoMask && D == 128) {
+        attr_err = cudaFuncSetAttribute(prefill_kernel<128, kNoMask, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)Cfg<128>::kSmemBytes);
         if (attr_err != cudaSuccess) return (int)attr_err;
       }
@@ -1122,7 +1217,7 @@ int launch(const TyrAttnPrefillArgs& a, float scale, int* status, cudaStream_t s
   p.lse_part = nullptr;
   p.item_table = nullptr;
   p.table_rounds = 0;
-  if (!kWindow && a.workspace != nullptr) {
+  if (kMask == kNoMask && a.workspace != nullptr) {
     const SplitPlan sp = split_plan(a, sm_count());
     if (sp.n_split > 0 && a.workspace_bytes >= sp.bytes && (reinterpret_cast<uintptr_t>(a.workspace) & 255) == 0) {
       p.n_split = sp.n_split;
@@ -1135,7 +1230,7 @@ int launch(const TyrAttnPrefillArgs& a, float scale, int* status, cudaStream_t s
       const int64_t part_stride[3] = {2ll * kBM * D, (int64_t)kBM * D, D};
       if ((rc = make_map(&top, p.o_part, sp.n_parts * sp.n_split, 2, kBM, D, part_stride))) return rc;
       const int grid = (int)std::min<long long>(items + (long long)sp.n_split * (sp.n_parts - 1), sm_count());
-      prefill_kernel<D, false, true, false><<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, p, top);
+      prefill_kernel<D, kNoMask, true, false><<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, p, top);
       count_launch();
       cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) return (int)e;
@@ -1161,13 +1256,13 @@ int launch(const TyrAttnPrefillArgs& a, float scale, int* status, cudaStream_t s
   // table (item_of_table).  Equal items gain nothing from it, and the tabled instantiation measured
   // 2.6 % slower than the plain one on them (Flux-shaped: 1128 vs 1158 TFLOP/s), so they stay static.
   // (and not for launches so large that the table itself would weigh: 4 bytes and a heap step per item)
-  if (!kWindow && D == 128 && p.causal && !p.snake && items >= 4ll * grid && items <= kMaxTabledItems &&
+  if (kMask == kNoMask && D == 128 && p.causal && !p.snake && items >= 4ll * grid && items <= kMaxTabledItems &&
       item_table_for(p, grid, st)) {
-    prefill_kernel<128, false, false, true><<<grid, kThreads, Cfg<128>::kSmemBytes, st>>>(tq, tk, tv, to, p, to);
+    prefill_kernel<128, kNoMask, false, true><<<grid, kThreads, Cfg<128>::kSmemBytes, st>>>(tq, tk, tv, to, p, to);
     count_launch();
     return (int)cudaGetLastError();
   }
-  prefill_kernel<D, kWindow, false, false><<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, p, to);
+  prefill_kernel<D, kMask, false, false><<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, p, to);
   count_launch();
   return (int)cudaGetLastError();
 }
@@ -1184,10 +1279,11 @@ long long prefill_split_workspace_bytes(const TyrAttnPrefillArgs& a) {
 }
 
 int launch_prefill_sm100(const TyrAttnPrefillArgs& a, float scale, int* status, cudaStream_t st) {
-  const bool win = a.window_size > 0 || a.key_mask != nullptr;
-  if (a.head_dim == 128) return win ? launch<128, true>(a, scale, status, st) : launch<128, false>(a, scale, status, st);
-  if (a.head_dim == 64) return win ? launch<64, true>(a, scale, status, st) : launch<64, false>(a, scale, status, st);
-  return -TYR_ATTN_ERR_HEAD_DIM;
+  if (a.head_dim != 64 && a.head_dim != 128) return -TYR_ATTN_ERR_HEAD_DIM;
+  const bool wide = a.head_dim == 128;
+  if (a.key_mask != nullptr) return wide ? launch<128, kKeyMask>(a, scale, status, st) : launch<64, kKeyMask>(a, scale, status, st);
+  if (a.window_size > 0) return wide ? launch<128, kWindowMask>(a, scale, status, st) : launch<64, kWindowMask>(a, scale, status, st);
+  return wide ? launch<128, kNoMask>(a, scale, status, st) : launch<64, kNoMask>(a, scale, status, st);
 }
 
 }  // namespace tyr
