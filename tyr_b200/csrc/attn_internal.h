@@ -36,6 +36,11 @@ inline cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// From this many query rows or keys on, the order of the sums behind a (batch, head)'s results is the same in
+// every causal launch, whatever else is in the batch: its bits are those of a call of its own.  Below it a launch
+// with too few work items for the SMs may cut a row's keys, or a key's query rows, over more of the device.
+constexpr int kOneOrderSeq = 2048;
+
 // Per-device state owned by api.cu.
 struct DeviceState {
   int* status = nullptr;  // device word the kernels' bounded waits OR into

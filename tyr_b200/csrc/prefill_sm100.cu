@@ -165,7 +165,11 @@ struct Bars {
   static constexpr int o_stage_free = o_staged + 1;       // [2] the TMA store of Q tile t's O has read the buffer
   static constexpr int rng_full = o_stage_free + 2;       // [2] padding mask: the item's range of KV tiles is known
   static constexpr int rng_empty = rng_full + 2;          // [2] every role has read it (producer, issuer, 8 softmax warps)
-  __device__ static constexpr uint32_t count(int i) {
+  // kHalves (never together with a padding mask) has two barriers of 8 softmax warps in their place
+  static constexpr int stat_full = rng_full;              // both slots' row maxima and sums are in shared memory
+  static constexpr int acc_free = rng_full + 1;           // both accumulators of the item have been read
+  __device__ static constexpr uint32_t count(int i, bool halves) {
+    if (halves && (i == stat_full || i == acc_free)) return 8u;
     if (i >= rng_empty) return 10u;
     return ((i >= p_half && i < p_half + 4) || i == o_staged) ? 4u : 1u;  // one arrival per softmax warp
   }
@@ -197,7 +201,7 @@ constexpr int kNoMask = 0, kWindowMask = 1, kKeyMask = 2;
 // the decode sat on the path between them: 24.4 -> 22.7 us).  With the long items of the D=128
 // workloads nothing is gained at the boundary, and that form of this function measured 3 % slower
 // there (1113 vs 1154 TFLOP/s, either order), so they keep the plain divisions.
-template <int kMask, bool kFast>
+template <int kMask, bool kFast, bool kHalves>
 __device__ __forceinline__ Item decode_item(int w, const PrefillParams& p) {
   Item it;
   const int n_groups = p.batch * p.n_kv_head;
@@ -232,6 +236,15 @@ __device__ __forceinline__ Item decode_item(int w, const PrefillParams& p) {
     hl = idx % heads_per_level;
   }
   const int nkv_total = (p.kv_seq + kBN - 1) / kBN;
+  if (kHalves) {
+    it.hq[0] = it.hq[1] = it.hkv * p.group + hl;
+    it.row[0] = it.row[1] = it.mblk * kBM;
+    const int n = p.causal ? min(nkv_total, it.mblk + 1) : nkv_total;
+    it.lo = 0;
+    it.n0 = (n + 1) >> 1;  // tiles 0, 2, ..
+    it.n1 = n >> 1;        // tiles 1, 3, ..
+    return it;
+  }
   int last0, last1;  // last KV tile (exclusive) under a causal mask
   if (p.pair_heads) {
     it.hq[0] = it.hkv * p.group + 2 * hl;
@@ -276,17 +289,17 @@ __device__ __forceinline__ int item_of_table(int it, const PrefillParams& p) {
 
 // Work item w of the launch: the items before p.split_from as they are, the ones from there on as
 // two to eight parts of their KV tiles each (non-causal launches only, so both Q tiles visit every tile).
-template <int D, int kMask, bool kSplit>
+template <int D, int kMask, bool kSplit, bool kHalves>
 __device__ __forceinline__ Item work_item(int w, const PrefillParams& p) {
   if (!kSplit || w < p.split_from) {
-    Item it = decode_item<kMask, D == 64>(w, p);
+    Item it = decode_item<kMask, D == 64, kHalves>(w, p);
     it.part_slot = -1;
     return it;
   }
   const int s = w - p.split_from;
   const int slot = p.by_parts.div(s);
   const int part = s - slot * p.n_parts;
-  Item it = decode_item<kMask, D == 64>(p.split_from + slot, p);
+  Item it = decode_item<kMask, D == 64, kHalves>(p.split_from + slot, p);
   const int n = it.n1;  // KV tiles of the whole item; part k covers tiles [k n / parts, (k + 1) n / parts)
   it.part_slot = part * p.n_split + slot;
   it.lo = part * n / p.n_parts;
@@ -421,7 +434,11 @@ __device__ __forceinline__ void exp_chunk(const uint32_t (&sr)[32], uint64_t sl2
 // kMask compiles the sliding window or the padding mask in (rows may then meet tiles in which they see no
 // key); the plain kernel carries none of those checks.
 // kSplit compiles the key-split of the last round in (work_item); the plain kernel has no trace of it.
-template <int D, int kMask, bool kSplit, bool kTabled>
+// kHalves: both Q-tile slots work on the same 128 query rows, slot 0 on the even and slot 1 on the odd KV tiles,
+// and the two softmax warpgroups merge their halves in the epilogue, each for half of the output columns
+// (both accumulators sit on the same tensor-memory lanes, so only the row maxima and sums cross).  For
+// launches with too few items for the SMs: an item of n KV tiles takes n / 2 steps of the same length.
+template <int D, int kMask, bool kSplit, bool kTabled, bool kHalves>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
@@ -447,7 +464,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   if (threadIdx.x == 0) {
     wait_ctl.abort = 0;
     wait_ctl.limit = p.wait_limit;
-    for (int i = 0; i < C::kNumBars; ++i) mbar_init(bar(i), B::count(i));
+    for (int i = 0; i < C::kNumBars; ++i) mbar_init(bar(i), B::count(i, kHalves));
     mbar_fence_init();
     tma_prefetch_desc(&tm_q);
     tma_prefetch_desc(&tm_k);
@@ -464,6 +481,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   const uint32_t tmem = tmem_slot;
   volatile WaitCtl* abortp = &wait_ctl;
 
+  // kHalves: row maximum and row sum of a slot's keys, [item & 1][slot][row]; it has no use for the staging buffer
+  float2* row_stat = reinterpret_cast<float2*>(smem_raw + (sO - raw));
   // Padding mask: cuts item number `it` of this CTA down to the tiles with a valid key, which the scan warp
   // has looked up.  Called once per item by the producing lane and by the issuing and softmax warps.
   auto cut_to_keys = [&](Item& im, int it, bool whole_warp) {
@@ -492,9 +511,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         for (int it = 0; ok; ++it) {
           const int w = kTabled ? item_of_table(it, p) : snake_item(it, total_items, p.snake);
           if (w < 0) break;
-          Item im = work_item<D, kMask, kSplit>(w, p);
+          Item im = work_item<D, kMask, kSplit, kHalves>(w, p);
 #pragma unroll
-          for (int t = 0; t < 2; ++t) {
+          for (int t = 0; t < (kHalves ? 1 : 2); ++t) {
             if (it > 0) ok = ok && mbar_wait(bar(B::q_empty + t), (it - 1) & 1, abortp);
             if (!ok) break;
             mbar_expect_tx(bar(B::q_full + t), C::kTileBytes);
@@ -527,9 +546,18 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           };
           if (ok) ok = cut_to_keys(im, it, false);
           if (ok) load_k(0);
-          for (int j = 0; j < im.n1 && ok; ++j) {
-            if (j + 1 < im.n1) load_k(j + 1);
-            load_v(j);
+          if (kHalves) {  // consumed in tile order, two tiles a step
+            const int n = im.n0 + im.n1;
+            if (ok && n > 1) load_k(1);
+            for (int j = 0; j < n && ok; ++j) {
+              load_v(j);
+              if (ok && j + 2 < n) load_k(j + 2);
+            }
+          } else {
+            for (int j = 0; j < im.n1 && ok; ++j) {
+              if (j + 1 < im.n1) load_k(j + 1);
+              load_v(j);
+            }
           }
         }
       }
@@ -548,9 +576,50 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         for (int it = 0; ok; ++it) {
           const int w = kTabled ? item_of_table(it, p) : snake_item(it, total_items, p.snake);
           if (w < 0) break;
-          Item im = work_item<D, kMask, kSplit>(w, p);
+          Item im = work_item<D, kMask, kSplit, kHalves>(w, p);
           if (!cut_to_keys(im, it, true)) break;
           const int n0 = im.n0, n1 = im.n1;
+          if (kHalves) {
+            // scores of tile number i of the item (slot i & 1); behind the last of them Q may go
+            const int n = n0 + n1;
+            auto score = [&](int i) {
+              const int s = kc % C::kKStages;
+              if (!mbar_wait(bar(B::k_full + s), (kc / C::kKStages) & 1, abortp)) return false;
+              tc_fence_after();
+              issue_qk<D>(issue, (i & 1) ? tS1 : tS0, q_desc0, umma_desc_lo(sK + s * C::kTileBytes, 16));
+              umma_commit_p(bar(B::s_full + (i & 1)), issue);
+              umma_commit_p(bar(B::k_empty + s), issue);
+              if (i == n - 1) umma_commit_p(bar(B::q_empty + 0), issue);
+              ++kc;
+              return true;
+            };
+            ok = mbar_wait(bar(B::q_full + 0), it & 1, abortp) && score(0);
+            if (ok && n > 1) ok = score(1);
+            // the first accumulating products overwrite what the previous item's epilogue reads
+            if (ok && it > 0) ok = mbar_wait(bar(B::acc_free), (it - 1) & 1, abortp);
+            for (int i = 0; i < n && ok; ++i) {
+              const int t = i & 1, vs = vc % C::kVStages, ph = (t ? pc1 : pc0) & 1;
+              const uint32_t tSt = t ? tS1 : tS0, tOt = t ? tO1 : tO0;
+              const uint32_t v_smem = umma_desc_lo(sV + vs * C::kTileBytes, C::kBoxBytes);
+              ok = mbar_wait(bar(B::v_full + vs), (vc / C::kVStages) & 1, abortp) &&
+                   mbar_wait(bar(B::p_half + t), ph, abortp);
+              if (!ok) break;
+              tc_fence_after();
+              issue_pv<D>(issue, tOt, tSt, v_smem, i > 1, 0);
+              ok = mbar_wait(bar(B::p_full + t), ph, abortp);
+              if (!ok) break;
+              tc_fence_after();
+              issue_pv<D>(issue, tOt, tSt, v_smem, true, 1);
+              umma_commit_p(bar(B::v_empty + vs), issue);
+              ++vc;
+              if (t) ++pc1;
+              else ++pc0;
+              if (i + 2 < n) ok = score(i + 2);
+            }
+            // one barrier for both accumulators: everything issued for the item is done
+            umma_commit_p(bar(B::o_full + 0), issue);
+            continue;
+          }
           ok = mbar_wait(bar(B::q_full + 0), it & 1, abortp) && mbar_wait(bar(B::q_full + 1), it & 1, abortp) &&
                mbar_wait(bar(B::k_full + kc % C::kKStages), (kc / C::kKStages) & 1, abortp);
           if (!ok) break;
@@ -634,7 +703,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       for (int it = 0; ok; ++it) {
         const int w = kTabled ? item_of_table(it, p) : snake_item(it, total_items, p.snake);
         if (w < 0) break;
-        const Item im = work_item<D, kMask, kSplit>(w, p);
+        const Item im = work_item<D, kMask, kSplit, kHalves>(w, p);
         const int4 cut = valid_tiles(p.key_mask + im.b * p.key_mask_stride, p.kv_seq, im.lo, im.n0, im.n1);
         if (it >= 2) ok = __all_sync(0xffffffffu, mbar_wait(bar(B::rng_empty + (it & 1)), ((it >> 1) - 1) & 1, abortp));
         if (!ok) break;
@@ -651,13 +720,13 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       // sends it out with one tiled TMA store per 64 columns and frees the buffer once the store
       // has read it.  Use number u = 2 item + tile; the uses are strictly ordered: a tile stages
       // only after the store of the use before it (the other tile's) has read the buffer.
-      if (lane == 0 && C::kStageO) {
+      if (lane == 0 && C::kStageO && !kHalves) {
         bool ok = true;
         int u = 0;
         for (int it = 0; ok; ++it) {
           const int w = kTabled ? item_of_table(it, p) : snake_item(it, total_items, p.snake);
           if (w < 0) break;
-          const Item im = work_item<D, kMask, kSplit>(w, p);
+          const Item im = work_item<D, kMask, kSplit, kHalves>(w, p);
 #pragma unroll
           for (int t = 0; t < 2; ++t, ++u) {
             ok = mbar_wait(bar(B::o_staged), u & 1, abortp);
@@ -692,22 +761,22 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     const uint32_t tS = tmem + lane_addr + C::kTmemS + t * kBN;
     const uint32_t tO = tmem + lane_addr + C::kTmemO + t * D;
     const float sl2 = p.scale_log2;
-    constexpr bool kRefByRow = kMask != kNoMask;  // rows may meet tiles in which they see no key
+    constexpr bool kRefByRow = kMask != kNoMask || kHalves;  // rows may meet tiles in which they see no key
     bool ok = true;
     int sc = 0;  // score tiles of this Q-tile slot processed so far, over all items
 
     for (int it = 0; ok; ++it) {
       const int w = kTabled ? item_of_table(it, p) : snake_item(it, total_items, p.snake);
       if (w < 0) break;
-      Item im = work_item<D, kMask, kSplit>(w, p);
+      Item im = work_item<D, kMask, kSplit, kHalves>(w, p);
       if (!cut_to_keys(im, it, true)) break;
       const int row = (t ? im.row[1] : im.row[0]) + r;  // query index
       const int hq = t ? im.hq[1] : im.hq[0];
       // the KV tiles by their first key (kRefByRow) or by number: the former keeps registers free where the
       // range comes from memory, the latter measured 4 % faster in the plain instantiation at D = 64
-      const int n_t = t ? im.n1 : im.n0;
-      const int j_begin = kRefByRow ? im.lo * kBN : 0, j_end = kRefByRow ? (im.lo + n_t) * kBN : n_t;
-      const int j_step = kRefByRow ? kBN : 1;
+      const int n_t = kHalves ? im.n0 + im.n1 : t ? im.n1 : im.n0;
+      const int j_begin = kRefByRow ? (im.lo + (kHalves ? t : 0)) * kBN : 0, j_end = kRefByRow ? (im.lo + n_t) * kBN : n_t;
+      const int j_step = kRefByRow ? (kHalves ? 2 * kBN : kBN) : 1;
       float m_ref = -INFINITY, l = 0.f;
 
       for (int j = j_begin; j < j_end; j += j_step, ++sc) {
@@ -817,6 +886,59 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         if (lane == 0) mbar_arrive(bar(B::p_full + t));
       }
       if (!ok) break;
+
+      if (kHalves) {
+        // epilogue: the two slots' halves of the keys, O = (w_0 O_0 + w_1 O_1) / (w_0 l_0 + w_1 l_1) with
+        // w_t = 2^((m_t - m) scale log2 e); this warpgroup writes half of the columns.  The statistics'
+        // buffer is used again two items on: a warp gets there only through the next item's barrier,
+        // on which every warp arrives after it has read this item's.
+        row_stat[((it & 1) * 2 + t) * kBM + r] = make_float2(m_ref, l);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(B::stat_full));
+        ok = mbar_wait(bar(B::stat_full), it & 1, abortp) && mbar_wait(bar(B::o_full + 0), it & 1, abortp);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        const float2 s0 = row_stat[(it & 1) * 2 * kBM + r], s1 = row_stat[((it & 1) * 2 + 1) * kBM + r];
+        const bool two = im.n1 > 0;  // one KV tile: slot 1 has no accumulator (whatever its columns hold is dropped)
+        const float m = fmaxf(s0.x, s1.x);
+        const float e0 = ex2_approx((s0.x - m) * sl2);
+        const float e1 = s1.x == -INFINITY ? 0.0f : ex2_approx((s1.x - m) * sl2);
+        const float sum = e0 * s0.y + e1 * s1.y, inv = 1.0f / sum;
+        const float w0 = e0 * inv, w1 = e1 * inv;
+        const uint32_t tO0 = tmem + lane_addr + C::kTmemO, tO1 = tO0 + D;
+        __nv_bfloat16* orow = p.o + im.b * p.o_stride_b + hq * p.o_stride_h + (int64_t)row * p.o_stride_s;
+#pragma unroll
+        for (int cc = 0; cc < D / 64; ++cc) {
+          const int c = t * (D / 64) + cc;
+          uint32_t a[32], b[32];
+          tmem_ld32(tO0 + c * 32, a);
+          tmem_ld32(tO1 + c * 32, b);
+          tmem_wait_ld();
+          tmem_ld_ready(a);
+          tmem_ld_ready(b);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            const float x = __uint_as_float(a[i]) * w0;
+            a[i] = __float_as_uint(two ? fmaf(__uint_as_float(b[i]), w1, x) : x);
+          }
+#pragma unroll
+          for (int q4 = 0; q4 < 4; ++q4) {
+            uint4 wv;
+            wv.x = pack_bf16x2(__uint_as_float(a[q4 * 8 + 0]), __uint_as_float(a[q4 * 8 + 1]));
+            wv.y = pack_bf16x2(__uint_as_float(a[q4 * 8 + 2]), __uint_as_float(a[q4 * 8 + 3]));
+            wv.z = pack_bf16x2(__uint_as_float(a[q4 * 8 + 4]), __uint_as_float(a[q4 * 8 + 5]));
+            wv.w = pack_bf16x2(__uint_as_float(a[q4 * 8 + 6]), __uint_as_float(a[q4 * 8 + 7]));
+            if (row < p.q_seq) *reinterpret_cast<uint4*>(orow + c * 32 + q4 * 8) = wv;
+          }
+        }
+        if (t == 0 && p.lse != nullptr && row < p.q_seq)
+          p.lse[im.b * p.lse_stride_b + hq * p.lse_stride_h + row] = 0.6931471805599453f * (m * sl2 + lg2_approx(sum));
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(B::acc_free));
+        continue;
+      }
 
       // epilogue: O_t / l -> bf16 -> the staging buffer in the 128-byte-swizzled box layout of the
       // tensor map (each thread owns one row; a warp's 16-byte pieces of 32 rows land on distinct
@@ -981,6 +1103,7 @@ int encode_map(CUtensorMap* m, const void* ptr, int batch, int heads, int seq, i
 // equal items on 148 SMs: 36 + 18 tile steps instead of 36 + 36).  The parts leave normalised
 // partial outputs in the caller's workspace and prefill_split_merge_kernel combines them.
 constexpr int kMaxSplitParts = 8;
+constexpr long long kOneChunkBytes = 96ll << 20;  // K and V that stay in L2 (126 MB) together
 struct SplitPlan {
   long long items;  // work items before any split
   int n_split;      // items of the last round to split (0: none)
@@ -1009,6 +1132,26 @@ SplitPlan split_plan(const TyrAttnPrefillArgs& a, int n_sm) {
   return sp;
 }
 
+// Whether the two Q-tile slots of a CTA should share 128 query rows and split their keys (kHalves): in a
+// launch of at most one round of work items, whose time is that of its longest item, when the CTA with the
+// most work then has less.  In halves of a KV-tile step, an item boundary counted as one, with the merge as
+// two.  One prompt of 517 rows, 32 heads of 128: 80 items of up to 5 steps become 160 of up to 3, 16.4 ->
+// 14.4 us; 1024 rows, 16 heads 22.5 -> 16.4 us; 40 rows on 700 keys 17.2 -> 12.3 us.
+bool halves_pay(const TyrAttnPrefillArgs& a, int n_sm) {
+  if (a.window_size > 0 || a.key_mask != nullptr) return false;
+  const int nkv = (a.kv_seq + kBN - 1) / kBN, n_mblk = (a.q_seq + kBM - 1) / kBM;
+  const long long per_level = (long long)a.n_head * a.batch, items = per_level * n_mblk;
+  if (a.q_seq >= kOneOrderSeq || a.kv_seq >= kOneOrderSeq) return false;
+  if (items > 2ll * n_sm || split_plan(a, n_sm).items > n_sm) return false;
+  auto tiles = [&](long long w) {  // KV tiles of item w, longest first
+    return a.is_causal ? std::min<int>(nkv, n_mblk - (int)(w / per_level)) : nkv;
+  };
+  auto cost = [&](long long w) { return 2 * ((tiles(w) + 1) / 2) + 2; };
+  int busiest = cost(0);
+  for (long long w = n_sm; w < items; ++w) busiest = std::max(busiest, cost(w) + cost(2ll * n_sm - 1 - w));  // mirrored round
+  return busiest < 2 * tiles(0) + 1;
+}
+
 // O = sum_i w_i O_i with w_i = exp(LSE_i - LSE), LSE = log sum_i exp LSE_i: the merge of
 // Tyr/GPU/Kernels/RingAttn.lean:164-180 over the parts of a split item.  16 bytes of a row per lane.
 template <int D>
@@ -1021,7 +1164,7 @@ __global__ void __launch_bounds__(256) prefill_split_merge_kernel(const PrefillP
   const int col = (lane % kLanesPerRow) * 8;
   const int r = id & (kBM - 1), t = (id >> 7) & 1, slot = id >> 8;
   if (slot >= p.n_split) return;
-  const Item im = decode_item<kNoMask, true>(p.split_from + slot, p);
+  const Item im = decode_item<kNoMask, true, false>(p.split_from + slot, p);
   const int row = im.row[t] + r;
   if (row >= p.q_seq) return;
   const int hq = im.hq[t];
@@ -1143,17 +1286,22 @@ int launch(const TyrAttnPrefillArgs& a, float scale, int* status, cudaStream_t s
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -TYR_ATTN_ERR_NO_DEVICE;
     if (!attr_set[dev].load(std::memory_order_acquire)) {
-      cudaError_t attr_err = cudaFuncSetAttribute(prefill_kernel<D, kMask, false, false>,
+      cudaError_t attr_err = cudaFuncSetAttribute(prefill_kernel<D, kMask, false, false, false>,
                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   (int)C::kSmemBytes);
       if (attr_err != cudaSuccess) return (int)attr_err;
       if (kMask == kNoMask) {
-        attr_err = cudaFuncSetAttribute(prefill_kernel<D, kNoMask, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        attr_err = cudaFuncSetAttribute(prefill_kernel<D, kNoMask, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)C::kSmemBytes);
         if (attr_err != cudaSuccess) return (int)attr_err;
       }
+      if (kMask == kNoMask) {
+        attr_err = cudaFuncSetAttribute(prefill_kernel<D, kNoMask, false, false, true>,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmemBytes);
+        if (attr_err != cudaSuccess) return (int)attr_err;
+      }
       if (kMask == kNoMask && D == 128) {
-        attr_err = cudaFuncSetAttribute(prefill_kernel<128, kNoMask, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        attr_err = cudaFuncSetAttribute(prefill_kernel<128, kNoMask, false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)Cfg<128>::kSmemBytes);
         if (attr_err != cudaSuccess) return (int)attr_err;
       }
@@ -1167,11 +1315,19 @@ int launch(const TyrAttnPrefillArgs& a, float scale, int* status, cudaStream_t s
   p.o_stride_s = a.o_stride[2];
   p.n_head = a.n_head;
   p.batch = a.batch;
+  // a launch whose last round is split gets that instead: parts on several CTAs
+  SplitPlan sp{0, 0, 0, 0};
+  if (kMask == kNoMask && a.workspace != nullptr) {
+    sp = split_plan(a, sm_count());
+    if (a.workspace_bytes < sp.bytes || (reinterpret_cast<uintptr_t>(a.workspace) & 255) != 0) sp.n_split = 0;
+  }
+  const bool halves = kMask == kNoMask && sp.n_split == 0 &&
+                      4ll * a.kv_seq * D * a.batch * a.n_kv_head <= kOneChunkBytes && halves_pay(a, sm_count());
   {
     const int group = a.n_head / a.n_kv_head;
     // pair two heads of a KV head when that removes idle slots: causal masks, short query blocks
-    p.pair_heads = (group % 2 == 0 && (a.is_causal || a.window_size > 0 || a.q_seq <= kBM)) ? 1 : 0;
-    p.n_mblk = p.pair_heads ? (a.q_seq + kBM - 1) / kBM : (a.q_seq + 2 * kBM - 1) / (2 * kBM);
+    p.pair_heads = (!halves && group % 2 == 0 && (a.is_causal || a.window_size > 0 || a.q_seq <= kBM)) ? 1 : 0;
+    p.n_mblk = (p.pair_heads || halves) ? (a.q_seq + kBM - 1) / kBM : (a.q_seq + 2 * kBM - 1) / (2 * kBM);
     p.items_per_group = p.n_mblk * (p.pair_heads ? group / 2 : group);
   }
   p.n_kv_head = a.n_kv_head;
@@ -1182,7 +1338,7 @@ int launch(const TyrAttnPrefillArgs& a, float scale, int* status, cudaStream_t s
     // the same time on K/V that is still in L2, and plain round-robin keeps them close.
     const long long group_bytes = std::max<long long>(2ll * a.kv_seq * D * 2, 1);
     const long long n_groups = (long long)a.batch * a.n_kv_head;
-    const bool all_fit = group_bytes * n_groups <= (96ll << 20);
+    const bool all_fit = group_bytes * n_groups <= kOneChunkBytes;
     const long long g = all_fit ? n_groups : std::max<long long>((48ll << 20) / group_bytes, 1);
     p.groups_per_chunk = (int)std::min<long long>(g, n_groups);
     p.snake = all_fit ? 1 : 0;
@@ -1217,39 +1373,36 @@ int launch(const TyrAttnPrefillArgs& a, float scale, int* status, cudaStream_t s
   p.lse_part = nullptr;
   p.item_table = nullptr;
   p.table_rounds = 0;
-  if (kMask == kNoMask && a.workspace != nullptr) {
-    const SplitPlan sp = split_plan(a, sm_count());
-    if (sp.n_split > 0 && a.workspace_bytes >= sp.bytes && (reinterpret_cast<uintptr_t>(a.workspace) & 255) == 0) {
-      p.n_split = sp.n_split;
-      p.n_parts = sp.n_parts;
-      p.by_parts = make_fastdiv(sp.n_parts);
-      p.split_from = (int)(items - sp.n_split);
-      p.o_part = static_cast<__nv_bfloat16*>(a.workspace);
-      p.lse_part = reinterpret_cast<float*>(p.o_part + (size_t)sp.n_split * sp.n_parts * 2 * kBM * D);
-      CUtensorMap top;
-      const int64_t part_stride[3] = {2ll * kBM * D, (int64_t)kBM * D, D};
-      if ((rc = make_map(&top, p.o_part, sp.n_parts * sp.n_split, 2, kBM, D, part_stride))) return rc;
-      const int grid = (int)std::min<long long>(items + (long long)sp.n_split * (sp.n_parts - 1), sm_count());
-      prefill_kernel<D, kNoMask, true, false><<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, p, top);
-      count_launch();
-      cudaError_t e = cudaGetLastError();
-      if (e != cudaSuccess) return (int)e;
-      // programmatic stream serialisation: the merge's launch latency hides behind the kernel's tail
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(sp.n_split * 256 / (8 * (32 / (D / 8))));   // 256 rows per item, 8 warps of 32 / (D / 8) rows
-      cfg.blockDim = dim3(256);
-      cfg.dynamicSmemBytes = 0;
-      cfg.stream = st;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-      attr[0].val.programmaticStreamSerializationAllowed = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      e = cudaLaunchKernelEx(&cfg, prefill_split_merge_kernel<D>, p);
-      count_launch();
-      if (e == cudaSuccess) e = cudaGetLastError();
-      return (int)e;
-    }
+  if (sp.n_split > 0) {
+    p.n_split = sp.n_split;
+    p.n_parts = sp.n_parts;
+    p.by_parts = make_fastdiv(sp.n_parts);
+    p.split_from = (int)(items - sp.n_split);
+    p.o_part = static_cast<__nv_bfloat16*>(a.workspace);
+    p.lse_part = reinterpret_cast<float*>(p.o_part + (size_t)sp.n_split * sp.n_parts * 2 * kBM * D);
+    CUtensorMap top;
+    const int64_t part_stride[3] = {2ll * kBM * D, (int64_t)kBM * D, D};
+    if ((rc = make_map(&top, p.o_part, sp.n_parts * sp.n_split, 2, kBM, D, part_stride))) return rc;
+    const int grid = (int)std::min<long long>(items + (long long)sp.n_split * (sp.n_parts - 1), sm_count());
+    prefill_kernel<D, kNoMask, true, false, false><<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, p, top);
+    count_launch();
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return (int)e;
+    // programmatic stream serialisation: the merge's launch latency hides behind the kernel's tail
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(sp.n_split * 256 / (8 * (32 / (D / 8))));   // 256 rows per item, 8 warps of 32 / (D / 8) rows
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = 0;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, prefill_split_merge_kernel<D>, p);
+    count_launch();
+    if (e == cudaSuccess) e = cudaGetLastError();
+    return (int)e;
   }
   const int grid = (int)std::min<long long>(items, sm_count());
   // Items of unequal length in several L2-sized chunks and many rounds: deal them to the CTAs by a
@@ -1258,11 +1411,16 @@ int launch(const TyrAttnPrefillArgs& a, float scale, int* status, cudaStream_t s
   // (and not for launches so large that the table itself would weigh: 4 bytes and a heap step per item)
   if (kMask == kNoMask && D == 128 && p.causal && !p.snake && items >= 4ll * grid && items <= kMaxTabledItems &&
       item_table_for(p, grid, st)) {
-    prefill_kernel<128, kNoMask, false, true><<<grid, kThreads, Cfg<128>::kSmemBytes, st>>>(tq, tk, tv, to, p, to);
+    prefill_kernel<128, kNoMask, false, true, false><<<grid, kThreads, Cfg<128>::kSmemBytes, st>>>(tq, tk, tv, to, p, to);
     count_launch();
     return (int)cudaGetLastError();
   }
-  prefill_kernel<D, kMask, false, false><<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, p, to);
+  if (halves) {
+    prefill_kernel<D, kNoMask, false, false, true><<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, p, to);
+    count_launch();
+    return (int)cudaGetLastError();
+  }
+  prefill_kernel<D, kMask, false, false, false><<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, p, to);
   count_launch();
   return (int)cudaGetLastError();
 }
