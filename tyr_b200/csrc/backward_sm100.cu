@@ -33,12 +33,16 @@
 // Warps of both: 0 TMA producer, 1 MMA issuer, 2 TMEM allocation, 4-11 elementwise + epilogue, two
 // warps per TMEM lane quarter (thread = row), each on one half of the score columns and of the
 // output columns.  Units are sorted by decreasing work and dealt to the CTAs in mirrored rounds.
+// The three launches overlap (launch_overlapped): each sets up while the one before drains, and the dQ kernel,
+// which needs the row statistics only, takes every SM that the dK/dV kernel leaves or does not fill.  64 x 6
+// heads of 256 rows x 64: 65.9 -> 59.2 us; one prompt of 512 rows, 32/8 heads of 128, with its forward 69 -> 53 us.
 // Every wait is bounded and reports through the per-device status word, as in the forward.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
 #include <algorithm>
 #include <atomic>
+#include <utility>
 
 #include "attn_internal.h"
 #include "ptx_sm100.cuh"
@@ -100,6 +104,7 @@ struct BwdParams {
   float sl2, scale;
   int* status;
   long long wait_limit;  // cycles any single barrier wait may take before the CTA gives up
+  int wait_first;        // dQ kernel: dQ overlaps an input, so the dK/dV kernel has to be through
 };
 
 constexpr uint32_t kBwdDescHi = umma_desc_hi(1024);
@@ -214,6 +219,10 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
   volatile WaitCtl* abortp = &wait_ctl;
+  // the row statistics (and everything before them in the stream) are complete from here on; the dQ kernel,
+  // which needs nothing of this one, may take the SMs that this one leaves or does not fill
+  grid_dependency_wait();
+  grid_launch_dependents();
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
@@ -624,6 +633,9 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
   volatile WaitCtl* abortp = &wait_ctl;
+  // Every CTA of the grid before has passed its own wait for the row statistics: the inputs are complete.  That
+  // grid may still be running and reading the inputs, so an output that overlaps one of them waits.
+  if (p.wait_first) grid_dependency_wait();
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
@@ -850,6 +862,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     tc_fence_after();
     tmem_dealloc(tmem, C::kTmemCols);
   }
+  grid_dependency_wait();  // this grid is complete only when the dK/dV kernel is: what follows sees all three gradients
 }
 
 // Row statistics of the backward: one group of D/8 lanes per query row, 16-byte loads.
@@ -861,6 +874,8 @@ bwd_rowstats_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __
                     int64_t os_h, int64_t os_s, int64_t ds_b, int64_t ds_h, int64_t ds_s, float scale,
                     int64_t total_rows) {
   constexpr int kLanes = D / 8;  // lanes per row
+  grid_launch_dependents();      // the dK/dV kernel may set up; it waits for this grid itself
+  grid_dependency_wait();
   const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kLanes;  // padded row index
   const int sub = threadIdx.x % kLanes;
   if (slot >= total_rows) return;
@@ -924,12 +939,13 @@ int launch_bwd(const TyrAttnBackwardArgs& a, float scale, int* status, cudaStrea
     const int64_t threads = padded_rows * kLanes;
     const int64_t blocks = (threads + 255) / 256;
     if (blocks > 0x7fffffffLL) return -TYR_ATTN_ERR_TOO_LARGE;
-    bwd_rowstats_kernel<D><<<(unsigned)blocks, 256, 0, st>>>(
+    cudaError_t e = launch_overlapped(
+        bwd_rowstats_kernel<D>, dim3((unsigned)blocks), dim3(256), 0, st, 1,
         static_cast<const __nv_bfloat16*>(a.o), static_cast<const __nv_bfloat16*>(a.d_o), a.lse, neg_lse2,
         neg_delta_s, a.n_head, a.q_seq, sq_pad, a.o_stride[0], a.o_stride[1], a.o_stride[2], a.do_stride[0],
         a.do_stride[1], a.do_stride[2], scale, padded_rows);
     count_launch();
-    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return (int)e;
   }
 
@@ -971,9 +987,11 @@ int launch_bwd(const TyrAttnBackwardArgs& a, float scale, int* status, cudaStrea
     p.out1_stride[i] = a.dk_stride[i];
     p.out2_stride[i] = a.dv_stride[i];
   }
-  bwd_dkdv_kernel<D><<<(unsigned)std::min<long long>(grid_kv, sms), kBwdThreads, C::kSmemBytes, st>>>(tk, tv, tq, tdo, p);
+  p.wait_first = 0;
+  cudaError_t e = launch_overlapped(bwd_dkdv_kernel<D>, dim3((unsigned)std::min<long long>(grid_kv, sms)), dim3(kBwdThreads),
+                                    C::kSmemBytes, st, 1, tk, tv, tq, tdo, p);
   count_launch();
-  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
 
   p.out1 = static_cast<__nv_bfloat16*>(a.d_q);
@@ -982,9 +1000,20 @@ int launch_bwd(const TyrAttnBackwardArgs& a, float scale, int* status, cudaStrea
     p.out1_stride[i] = a.dq_stride[i];
     p.out2_stride[i] = 0;
   }
-  bwd_dq_kernel<D><<<(unsigned)std::min<long long>(grid_q, sms), kBwdThreads, DqCfg<D>::kSmemBytes, st>>>(tq, tdo, tk, tv, p);
+  {
+    auto span = [&](const void* ptr, int heads, int seq, const int64_t* stride) {
+      const char* lo = static_cast<const char*>(ptr);
+      return std::make_pair(lo, lo + 2 * ((a.batch - 1) * stride[0] + (heads - 1) * stride[1] + (seq - 1) * stride[2] + D));
+    };
+    const auto out = span(a.d_q, a.n_head, a.q_seq, a.dq_stride);
+    for (const auto& in : {span(a.q, a.n_head, a.q_seq, a.q_stride), span(a.d_o, a.n_head, a.q_seq, a.do_stride),
+                           span(a.k, a.n_kv_head, a.kv_seq, a.k_stride), span(a.v, a.n_kv_head, a.kv_seq, a.v_stride)})
+      if (out.first < in.second && in.first < out.second) p.wait_first = 1;
+  }
+  e = launch_overlapped(bwd_dq_kernel<D>, dim3((unsigned)std::min<long long>(grid_q, sms)), dim3(kBwdThreads),
+                        DqCfg<D>::kSmemBytes, st, 1, tq, tdo, tk, tv, p);
   count_launch();
-  return (int)cudaGetLastError();
+  return (int)(e != cudaSuccess ? e : cudaGetLastError());
 }
 
 }  // namespace
