@@ -59,7 +59,7 @@ struct BCfg {
   static constexpr int kBoxes = D / 64;                // 128-byte boxes per row
   static constexpr uint32_t kBoxBytes = 128u * 128u;   // 128 rows x 128 B
   static constexpr uint32_t kTileBytes = kBoxes * kBoxBytes;
-  static constexpr int kStages = 2;
+  static constexpr int kStages = (D == 64) ? 4 : 2;
   static constexpr uint32_t kRes1 = 0, kRes2 = kTileBytes;
   static constexpr uint32_t kStr = 2 * kTileBytes;     // stage s: tile 1 at kStr + 2 s T, tile 2 one T further
   // per stage: the streamed query block's 128 row statistics, two fp32 vectors (mode 0 only)
@@ -68,24 +68,30 @@ struct BCfg {
   static constexpr uint32_t kBarOff = kStatOff + kStages * kStatBytes;
   // barriers
   static constexpr int res_full = 0;                   // resident pair landed
-  static constexpr int str_full = 1;                   // [2] streamed pair landed
-  static constexpr int str_empty = 3;                  // [2] accumulating products have read the pair
-  static constexpr int s_full = 5;                     // S^T in tensor memory
-  static constexpr int p_full = 6;                     // P^T written (one arrival per elementwise warp)
-  static constexpr int acc_full = 7;                   // last accumulating product done
-  static constexpr int pair = 8;                       // [4] per lane quarter: both warps hold their score columns
+  static constexpr int str_full = 1;                   // [kStages] streamed pair landed
+  static constexpr int str_empty = 1 + kStages;        // [kStages] accumulating products have read the pair
+  static constexpr int kB = 1 + 2 * kStages;
+  static constexpr int s_full = kB + 0;                // S^T in tensor memory
+  static constexpr int p_full = kB + 1;                // P^T written (one arrival per elementwise warp)
+  static constexpr int acc_full = kB + 2;              // last accumulating product done
+  static constexpr int pair = kB + 3;                  // [4] per lane quarter: both warps hold their score columns
                                                        //     in registers (P / dS overwrite each other's columns)
-  static constexpr int res_empty = 12;                 // the unit's last score products have read K and V
-  static constexpr int acc_free = 13;                  // the epilogue has read dK and dV (8 warp arrivals)
-  static constexpr int ds_half = 14;                   // dS^T of score columns 0..63 written (8 warp arrivals)
-  static constexpr int ds_full = 15;                   // dS^T of score columns 64..127 written (8 warp arrivals)
-  static constexpr int dp_full = 16;                   // dP^T in tensor memory
-  static constexpr int dp_taken = 17;                  // dP^T is in registers: its columns are free (8 warp arrivals)
-  static constexpr int kNumBars = 18;
+  static constexpr int res_empty = kB + 7;             // the unit's last score products have read K and V
+  static constexpr int acc_free = kB + 8;              // the epilogue has read dK and dV (8 warp arrivals)
+  static constexpr int ds_half = kB + 9;               // dS^T of score columns 0..63 written (8 warp arrivals)
+  static constexpr int ds_full = kB + 10;              // dS^T of score columns 64..127 written (8 warp arrivals)
+  static constexpr int dp_full = kB + 11;              // dP^T in tensor memory
+  static constexpr int dp_taken = kB + 12;             // dP^T is in registers: its columns are free (8 warp arrivals)
+  static constexpr int kNumBars = kB + 13;
   static constexpr uint32_t kSmemBytes = kBarOff + kNumBars * 8 + 16 + 1024;  // + align slack
   static constexpr uint32_t kTmemCols = 512;
   static constexpr uint32_t kTmemS = 0, kTmemDP = 128, kTmemAcc1 = 256, kTmemAcc2 = 256 + D;
-  static_assert(256 + 2 * D <= 512, "tensor memory budget");
+  // D = 64 has a third score region: S^T alternates between the first two, dP^T has the third to itself.  The
+  // next pair's S^T is then there when the elementwise warps, which bound a pair at this head size, come for
+  // it (2 x 4096 rows, 32/8 heads: whole backward 637 -> 598 us).  Four stages because there is room.
+  static constexpr bool kThirdRegion = (D == 64);
+  static constexpr uint32_t kTmemR3 = 256 + 2 * D;
+  static_assert(kTmemR3 + (kThirdRegion ? 128 : 0) <= 512, "tensor memory budget");
   static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
 };
 
@@ -277,7 +283,11 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
       // bf16 overlays, P^T on its first 64 columns and dS^T on its last 64; the dP^T region is free as
       // soon as dP^T is in registers and takes S^T of pair g + 1, and when the accumulating products
       // of pair g have read the overlays their region takes dP^T of pair g + 1.
-      auto region = [&](int g, int which) { return tmem + (((g + which) & 1) ? C::kTmemDP : C::kTmemS); };
+      // With the third region (D = 64) dP^T is there, and S^T(g + 1) waits for nothing but its tiles.
+      auto region = [&](int g, int which) {
+        if (C::kThirdRegion && which) return tmem + C::kTmemR3;
+        return tmem + (((g + which) & 1) ? C::kTmemDP : C::kTmemS);
+      };
       auto score_s = [&](int g) {   // S^T = K Q^T of pair g
         const int s = g % C::kStages;
         if (!mbar_wait_q(bar(C::str_full + s), (g / C::kStages) & 1, abortp)) return false;
@@ -314,13 +324,19 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
           if (ok && i == 0 && rc > 0) ok = mbar_wait_q(bar(C::acc_free), (rc - 1) & 1, abortp);
           if (!ok) break;
           tc_fence_after();
+          if (C::kThirdRegion && i + 1 < w.n_iter) {
+            // S^T of the next pair: its region's overlays were read by the pair before this one.  Not earlier:
+            // it sets off the elementwise warps' next arrivals on the barriers waited for above.
+            ok = score_s(it + 1);
+            if (!ok) break;
+          }
           issue_acc<D>(issue, tA2, tP, do_mn, i > 0);
           // S^T of the next pair into the region dP^T has left
           if (i + 1 < w.n_iter) {
             ok = mbar_wait_q(bar(C::dp_taken), it & 1, abortp);
             if (!ok) break;
             tc_fence_after();
-            ok = score_s(it + 1);
+            if (!C::kThirdRegion) ok = score_s(it + 1);
             if (!ok) break;
           }
           // dK += dS^T Q, the first 64 query columns while the second 64 are still being formed
@@ -331,11 +347,12 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
           ok = mbar_wait_q(bar(C::ds_full), it & 1, abortp);
           if (!ok) break;
           tc_fence_after();
+          if (C::kThirdRegion && i + 1 < w.n_iter) score_dp(it + 1);  // (behind the last wait of this pair, as above)
           issue_acc<D>(issue, tA1, tDS, q_mn, true, 1);
           umma_commit_p(bar(C::str_empty + s), issue);
           if (i + 1 < w.n_iter) {
             // dP^T of the next pair into the region whose overlays the products above have read
-            score_dp(it + 1);
+            if (!C::kThirdRegion) score_dp(it + 1);
             // K and V are read by the score products only: after the unit's last pair of them
             // the producer may fetch the next unit's
             if (i + 2 == w.n_iter) umma_commit_p(bar(C::res_empty), issue);
@@ -363,7 +380,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
       for (int i = 0; i < w.n_iter; ++i, ++it) {
         // the score regions swap roles with every streamed pair (see the MMA issuer)
         const uint32_t tS = tmem + lane_addr + ((it & 1) ? C::kTmemDP : C::kTmemS);
-        const uint32_t tDP = tmem + lane_addr + ((it & 1) ? C::kTmemS : C::kTmemDP);
+        const uint32_t tDP = tmem + lane_addr + (C::kThirdRegion ? C::kTmemR3 : (it & 1) ? C::kTmemS : C::kTmemDP);
         ok = mbar_wait_q(bar(C::s_full), it & 1, abortp);
         // the query columns' statistics landed with the streamed tiles: observe that barrier
         // directly (it completed before the products this warp was woken by were issued)
