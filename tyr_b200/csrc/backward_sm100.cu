@@ -42,7 +42,9 @@
 
 #include <algorithm>
 #include <atomic>
+#include <functional>
 #include <utility>
+#include <vector>
 
 #include "attn_internal.h"
 #include "ptx_sm100.cuh"
@@ -110,6 +112,7 @@ struct BwdParams {
   float sl2, scale;
   int* status;
   long long wait_limit;  // cycles any single barrier wait may take before the CTA gives up
+  int parts;             // dK/dV kernel: CTAs of a cluster that share a unit (1: none)
   int wait_first;        // dQ kernel: dQ overlaps an input, so the dK/dV kernel has to be through
 };
 
@@ -183,11 +186,20 @@ __device__ __forceinline__ KvUnit kv_unit(int u, const BwdParams& p) {
   return w;
 }
 
+// kCluster: the streamed pairs of a unit are dealt to the CTAs of a cluster (pair i to CTA i mod size), each with
+// the unit's K and V tiles, and their partial dK and dV are summed through distributed shared memory in
+// the order of the CTAs.  One unit per cluster, for launches with too few units for the SMs.
+struct UnitPart {
+  int rank, size;
+  __device__ __forceinline__ int pairs(int n) const { return (n - rank + size - 1) / size; }  // of a unit of n
+  __device__ __forceinline__ int pair(int i) const { return i * size + rank; }               // this CTA's i-th
+};
+
 // dK / dV kernel, persistent: CTA c works on units c, c + gridDim.x, ...  Rows = keys.  The K and V
 // tiles of the unit stay in shared memory (the next unit's are fetched as soon as the unit's last
 // score products have read them), Q and dO stream.  Barrier phases run on across units: every role
 // counts streamed tile pairs (`it`) and units with work (`rc`) for itself.
-template <int D>
+template <int D, bool kCluster>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                 const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
@@ -203,6 +215,14 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
   auto bar = [&](int i) { return sBar + 8u * i; };
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_units = p.n_kblk * p.n_kv_head * p.batch;
+  const int n_rounds = kCluster ? 1 : rounds_of(n_units);
+  const UnitPart part = {kCluster ? static_cast<int>(cluster_rank()) : 0, kCluster ? p.parts : 1};
+  auto unit_at = [&](int round) { return kCluster ? static_cast<int>(blockIdx.x) / part.size : unit_of_round(round, n_units); };
+  auto unit = [&](int u) {
+    KvUnit w = kv_unit(u, p);
+    if (kCluster) w.n_iter = part.pairs(w.n_iter);
+    return w;
+  };
 
   if (threadIdx.x == 0) {
     wait_ctl.abort = 0;
@@ -235,10 +255,10 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
     if (lane == 0) {
       bool ok = true;
       int it = 0, rc = 0;
-      for (int round = 0; round < rounds_of(n_units) && ok; ++round) {
-        const int u = unit_of_round(round, n_units);
+      for (int round = 0; round < n_rounds && ok; ++round) {
+        const int u = unit_at(round);
         if (u < 0) continue;
-        const KvUnit w = kv_unit(u, p);
+        const KvUnit w = unit(u);
         if (w.n_iter == 0) continue;
         if (rc > 0) ok = mbar_wait_q(bar(C::res_empty), (rc - 1) & 1, abortp);
         if (!ok) break;
@@ -252,7 +272,8 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
           const int s = it % C::kStages;
           if (it >= C::kStages) ok = mbar_wait_q(bar(C::str_empty + s), ((it / C::kStages) - 1) & 1, abortp);
           if (!ok) break;
-          const int hq = w.head * p.group + i / w.per_head, qblk = w.lo + i % w.per_head;
+          const int gi = kCluster ? part.pair(i) : i;
+          const int hq = w.head * p.group + gi / w.per_head, qblk = w.lo + gi % w.per_head;
           const uint32_t dst = base + C::kStr + s * 2 * C::kTileBytes;
           mbar_expect_tx(bar(C::str_full + s), 2 * C::kTileBytes + C::kStatBytes);
           {
@@ -303,10 +324,10 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
       };
       bool ok = true;
       int it = 0, rc = 0;
-      for (int round = 0; round < rounds_of(n_units) && ok; ++round) {
-        const int u = unit_of_round(round, n_units);
+      for (int round = 0; round < n_rounds && ok; ++round) {
+        const int u = unit_at(round);
         if (u < 0) continue;
-        const KvUnit w = kv_unit(u, p);
+        const KvUnit w = unit(u);
         if (w.n_iter == 0) continue;
         ok = mbar_wait_q(bar(C::res_full), rc & 1, abortp);
         if (ok) ok = score_s(it);
@@ -372,10 +393,10 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
     const uint64_t sl2x2 = pack_f32x2(p.sl2, p.sl2), scale2 = pack_f32x2(p.scale, p.scale);
     bool ok = true;
     int it = 0, rc = 0;
-    for (int round = 0; round < rounds_of(n_units) && ok; ++round) {
-      const int u = unit_of_round(round, n_units);
+    for (int round = 0; round < n_rounds && ok; ++round) {
+      const int u = unit_at(round);
       if (u < 0) continue;
-      const KvUnit w = kv_unit(u, p);
+      const KvUnit w = unit(u);
       const int row0 = w.blk * kT;
       for (int i = 0; i < w.n_iter; ++i, ++it) {
         // the score regions swap roles with every streamed pair (see the MMA issuer)
@@ -388,7 +409,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
-        const int col0 = (w.lo + i % w.per_head) * kT;  // first query of the score columns
+        const int col0 = (w.lo + (kCluster ? part.pair(i) : i) % w.per_head) * kT;  // first query of the score columns
         // under the causal mask a key row keeps the query columns with query >= key
         int c_first = p.causal ? row0 + r - col0 : 0;
         // sliding window: the key also drops out for queries with query - key >= window
@@ -497,6 +518,29 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
         if (!ok) break;
         tc_fence_after();
       }
+      if (kCluster) {
+        // partial dK and dV to shared memory, in the place of the streamed tiles, which have all been read:
+        // four columns of the 2 D of a row per 16 bytes, the 128 rows of those four side by side
+        float4* buf = reinterpret_cast<float4*>(smem_raw + (base - raw) + C::kStr);
+#pragma unroll
+        for (int cc = 0; cc < D / 32; ++cc) {
+          const int c = half * (D / 32) + cc;  // half 0: dK, half 1: dV
+          uint32_t o[32];
+          if (w.n_iter > 0) {
+            tmem_ld32(tmem + lane_addr + C::kTmemAcc1 + c * 32, o);
+            tmem_wait_ld();
+            tmem_ld_ready(o);
+          } else {
+#pragma unroll
+            for (int x = 0; x < 32; ++x) o[x] = 0u;
+          }
+#pragma unroll
+          for (int q4 = 0; q4 < 8; ++q4)
+            buf[(c * 8 + q4) * kT + r] = make_float4(__uint_as_float(o[q4 * 4]), __uint_as_float(o[q4 * 4 + 1]),
+                                                     __uint_as_float(o[q4 * 4 + 2]), __uint_as_float(o[q4 * 4 + 3]));
+        }
+        break;
+      }
       const int row = row0 + r;
       const bool row_ok = row < p.kv_seq;
 #pragma unroll
@@ -538,6 +582,32 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
 
   // ------------------------------------------------------------------ exit
   __syncwarp();
+  if (kCluster) {
+    // Every CTA sums its share of the rows over the cluster.  All threads come here, also after a wait
+    // that gave up (the sums are then as useless as the status says).
+    cluster_sync();
+    const KvUnit w = kv_unit(unit_at(0), p);
+    const int rows = kT / part.size, row0 = part.rank * rows;
+    const uint32_t buf = base + C::kStr;
+    // a group of 32 elements: 8 neighbouring column quadruples of 4 rows
+    for (int e = threadIdx.x; e < rows * (D / 2); e += kBwdThreads) {
+      const int g = e >> 5, r = row0 + (g % (rows / 4)) * 4 + (e & 3), c4 = (g / (rows / 4)) * 8 + ((e >> 2) & 7);
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int k = 0; k < part.size; ++k) {
+        const float4 v = cluster_ld_f32x4(cluster_map(buf + (c4 * kT + r) * 16, k));
+        acc.x += v.x;
+        acc.y += v.y;
+        acc.z += v.z;
+        acc.w += v.w;
+      }
+      const int row = w.blk * kT + r, which = c4 / (D / 4), col = (c4 % (D / 4)) * 4;
+      const int64_t* st = which ? p.out2_stride : p.out1_stride;
+      __nv_bfloat16* orow = (which ? p.out2 : p.out1) + w.b * st[0] + w.head * st[1] + (int64_t)row * st[2];
+      if (row < p.kv_seq)
+        *reinterpret_cast<uint2*>(orow + col) = make_uint2(pack_bf16x2(acc.x, acc.y), pack_bf16x2(acc.z, acc.w));
+    }
+    cluster_sync();  // no CTA's shared memory goes away while another still reads it
+  }
   tc_fence_before();
   __syncthreads();
   if (wait_ctl.abort != 0) {
@@ -922,6 +992,39 @@ bwd_rowstats_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __
   }
 }
 
+// CTAs that share a unit of the dK/dV kernel.  A launch of few units takes as long as its longest one (the
+// first keys are seen by every query row of every head of the group); several CTAs per unit cost a
+// cluster's merge and a CTA's set-up each, together about kMergePairs streamed pairs.  The number with the
+// shortest makespan, units dealt longest first, and only where it is a tenth shorter.  One prompt of 512 rows,
+// 32/8 heads: 32 units on 148 SMs; forward and backward 53 -> 41 us at D = 128, 43 -> 33 us at D = 64.
+constexpr int kMergePairs = 3;
+int unit_parts(const BwdParams& p, int sms) {
+  const long long units = (long long)p.n_kblk * p.n_kv_head * p.batch;
+  if (units >= 2ll * sms || p.q_seq >= kOneOrderSeq || p.kv_seq >= kOneOrderSeq) return 1;
+  long long best = 0;
+  int best_parts = 1;
+  for (int parts = 1; parts <= 8; parts *= 2) {
+    std::vector<long long> load(std::max(sms / parts, 1), 0);  // a min-heap over the clusters that run at once
+    auto later = std::greater<long long>();
+    for (int blk = 0; blk < p.n_kblk; ++blk) {
+      const int lo = p.causal ? std::min(blk, p.n_qblk) : 0;
+      const int hi = p.window > 0 ? std::min(p.n_qblk, (blk * kT + kT - 1 + p.window - 1) / kT + 1) : p.n_qblk;
+      const long long n = (long long)std::max(hi - lo, 0) * p.group;
+      for (int i = 0; i < p.n_kv_head * p.batch; ++i) {
+        std::pop_heap(load.begin(), load.end(), later);
+        load.back() += (n + parts - 1) / parts + (parts > 1 ? kMergePairs : 1);
+        std::push_heap(load.begin(), load.end(), later);
+      }
+    }
+    const long long span = *std::max_element(load.begin(), load.end());
+    if (parts == 1 || 10 * span < 9 * best) {
+      best = span;
+      best_parts = parts;
+    }
+  }
+  return best_parts;
+}
+
 template <int D>
 int launch_bwd(const TyrAttnBackwardArgs& a, float scale, int* status, cudaStream_t st) {
   using C = BCfg<D>;
@@ -942,8 +1045,10 @@ int launch_bwd(const TyrAttnBackwardArgs& a, float scale, int* status, cudaStrea
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -TYR_ATTN_ERR_NO_DEVICE;
     if (!attr_set[dev].load(std::memory_order_acquire)) {
-      cudaError_t e = cudaFuncSetAttribute(bwd_dkdv_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      cudaError_t e = cudaFuncSetAttribute(bwd_dkdv_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)C::kSmemBytes);
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(bwd_dkdv_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmemBytes);
       if (e == cudaSuccess)
         e = cudaFuncSetAttribute(bwd_dq_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)DqCfg<D>::kSmemBytes);
@@ -1005,8 +1110,12 @@ int launch_bwd(const TyrAttnBackwardArgs& a, float scale, int* status, cudaStrea
     p.out2_stride[i] = a.dv_stride[i];
   }
   p.wait_first = 0;
-  cudaError_t e = launch_overlapped(bwd_dkdv_kernel<D>, dim3((unsigned)std::min<long long>(grid_kv, sms)), dim3(kBwdThreads),
-                                    C::kSmemBytes, st, 1, tk, tv, tq, tdo, p);
+  p.parts = unit_parts(p, sms);
+  cudaError_t e = p.parts > 1
+                      ? launch_overlapped(bwd_dkdv_kernel<D, true>, dim3((unsigned)(grid_kv * p.parts)), dim3(kBwdThreads),
+                                          C::kSmemBytes, st, (unsigned)p.parts, tk, tv, tq, tdo, p)
+                      : launch_overlapped(bwd_dkdv_kernel<D, false>, dim3((unsigned)std::min<long long>(grid_kv, sms)),
+                                          dim3(kBwdThreads), C::kSmemBytes, st, 1, tk, tv, tq, tdo, p);
   count_launch();
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
