@@ -42,9 +42,7 @@
 
 #include <algorithm>
 #include <atomic>
-#include <functional>
 #include <utility>
-#include <vector>
 
 #include "attn_internal.h"
 #include "ptx_sm100.cuh"
@@ -995,8 +993,9 @@ bwd_rowstats_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __
 // CTAs that share a unit of the dK/dV kernel.  A launch of few units takes as long as its longest one (the
 // first keys are seen by every query row of every head of the group); several CTAs per unit cost a
 // cluster's merge and a CTA's set-up each, together about kMergePairs streamed pairs.  The number with the
-// shortest makespan, units dealt longest first, and only where it is a tenth shorter.  One prompt of 512 rows,
-// 32/8 heads: 32 units on 148 SMs; forward and backward 53 -> 41 us at D = 128, 43 -> 33 us at D = 64.
+// shortest time, taken as the longest unit or the average load of the clusters that run at once, and only
+// where it is a tenth shorter.  One prompt of 512 rows, 32/8 heads: 32 units on 148 SMs; forward and backward
+// 53 -> 41 us at D = 128, 43 -> 33 us at D = 64.
 constexpr int kMergePairs = 3;
 int unit_parts(const BwdParams& p, int sms) {
   const long long units = (long long)p.n_kblk * p.n_kv_head * p.batch;
@@ -1004,19 +1003,16 @@ int unit_parts(const BwdParams& p, int sms) {
   long long best = 0;
   int best_parts = 1;
   for (int parts = 1; parts <= 8; parts *= 2) {
-    std::vector<long long> load(std::max(sms / parts, 1), 0);  // a min-heap over the clusters that run at once
-    auto later = std::greater<long long>();
+    long long longest = 0, total = 0;
     for (int blk = 0; blk < p.n_kblk; ++blk) {
       const int lo = p.causal ? std::min(blk, p.n_qblk) : 0;
       const int hi = p.window > 0 ? std::min(p.n_qblk, (blk * kT + kT - 1 + p.window - 1) / kT + 1) : p.n_qblk;
       const long long n = (long long)std::max(hi - lo, 0) * p.group;
-      for (int i = 0; i < p.n_kv_head * p.batch; ++i) {
-        std::pop_heap(load.begin(), load.end(), later);
-        load.back() += (n + parts - 1) / parts + (parts > 1 ? kMergePairs : 1);
-        std::push_heap(load.begin(), load.end(), later);
-      }
+      const long long cost = (n + parts - 1) / parts + (parts > 1 ? kMergePairs : 1);
+      longest = std::max(longest, cost);
+      total += cost * p.n_kv_head * p.batch;
     }
-    const long long span = *std::max_element(load.begin(), load.end());
+    const long long span = std::max(longest, total * parts / sms);
     if (parts == 1 || 10 * span < 9 * best) {
       best = span;
       best_parts = parts;
