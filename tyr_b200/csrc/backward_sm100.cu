@@ -72,7 +72,7 @@ struct BCfg {
   static constexpr int str_empty = 1 + kStages;        // [kStages] accumulating products have read the pair
   static constexpr int kB = 1 + 2 * kStages;
   static constexpr int s_full = kB + 0;                // S^T in tensor memory
-  static constexpr int p_full = kB + 1;                // P^T written (one arrival per elementwise warp)
+  static constexpr int p_full = kB + 1;                // P^T written (one arrival per elementwise warp), its second half with kHalfP
   static constexpr int acc_full = kB + 2;              // last accumulating product done
   static constexpr int pair = kB + 3;                  // [4] per lane quarter: both warps hold their score columns
                                                        //     in registers (P / dS overwrite each other's columns)
@@ -82,7 +82,12 @@ struct BCfg {
   static constexpr int ds_full = kB + 10;              // dS^T of score columns 64..127 written (8 warp arrivals)
   static constexpr int dp_full = kB + 11;              // dP^T in tensor memory
   static constexpr int dp_taken = kB + 12;             // dP^T is in registers: its columns are free (8 warp arrivals)
-  static constexpr int kNumBars = kB + 13;
+  static constexpr int p_half = kB + 13;               // kHalfP: P^T of query columns 0..63 written (8 warp arrivals)
+  static constexpr int kNumBars = kB + 14;
+  // D = 128: P^T is handed over in two halves, so that dV of the first 64 query columns runs during the
+  // exponentials of the second 64.  The backward of 4096 rows, 32/8 heads 405.3 -> 399.0 us, of 8 x 2048 rows,
+  // 16/8 heads 487.3 -> 484.3; at D = 64, where the elementwise warps are the bound, the extra hand-over cost 0.3 %.
+  static constexpr bool kHalfP = (D == 128);
   static constexpr uint32_t kSmemBytes = kBarOff + kNumBars * 8 + 16 + 1024;  // + align slack
   static constexpr uint32_t kTmemCols = 512;
   static constexpr uint32_t kTmemS = 0, kTmemDP = 128, kTmemAcc1 = 256, kTmemAcc2 = 256 + D;
@@ -226,7 +231,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
     wait_ctl.abort = 0;
     wait_ctl.limit = p.wait_limit;
     for (int i = 0; i < C::kNumBars; ++i)
-      mbar_init(bar(i), (i == C::p_full || i == C::ds_half || i == C::ds_full || i == C::dp_taken || i == C::acc_free) ? 8u
+      mbar_init(bar(i), (i == C::p_half || i == C::p_full || i == C::ds_half || i == C::ds_full || i == C::dp_taken || i == C::acc_free) ? 8u
                         : (i >= C::pair && i < C::pair + 4) ? 2u : 1u);
     mbar_fence_init();
     tma_prefetch_desc(&tm_k);
@@ -337,19 +342,25 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
           const uint32_t tP = region(it, 0), tDS = tP + 64;
           const uint32_t q_mn = umma_desc_lo(t1, C::kBoxBytes), do_mn = umma_desc_lo(t1 + C::kTileBytes, C::kBoxBytes);
           // dV += P^T dO as soon as P^T is written (it is formed from S^T alone, ahead of dS^T)
-          ok = mbar_wait_q(bar(C::p_full), it & 1, abortp);
+          ok = mbar_wait_q(bar(C::kHalfP ? C::p_half : C::p_full), it & 1, abortp);
           // the unit's first accumulating products overwrite dK / dV: the previous unit's
           // epilogue must have read them
           if (ok && i == 0 && rc > 0) ok = mbar_wait_q(bar(C::acc_free), (rc - 1) & 1, abortp);
           if (!ok) break;
           tc_fence_after();
+          if (C::kHalfP) {
+            issue_acc<D>(issue, tA2, tP, do_mn, i > 0, 0);
+            ok = mbar_wait_q(bar(C::p_full), it & 1, abortp);
+            if (!ok) break;
+            tc_fence_after();
+          }
           if (C::kThirdRegion && i + 1 < w.n_iter) {
             // S^T of the next pair: its region's overlays were read by the pair before this one.  Not earlier:
             // it sets off the elementwise warps' next arrivals on the barriers waited for above.
             ok = score_s(it + 1);
             if (!ok) break;
           }
-          issue_acc<D>(issue, tA2, tP, do_mn, i > 0);
+          issue_acc<D>(issue, tA2, tP, do_mn, C::kHalfP || i > 0, C::kHalfP ? 1 : -1);
           // S^T of the next pair into the region dP^T has left
           if (i + 1 < w.n_iter) {
             ok = mbar_wait_q(bar(C::dp_taken), it & 1, abortp);
@@ -462,6 +473,12 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
             tc_fence_after();
           }
           tmem_st16(tS + c * 16, pk_p);
+          if (C::kHalfP && step == 0) {
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(C::p_half));
+          }
         }
         if (!ok) break;
         tmem_wait_st();
