@@ -480,6 +480,12 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
   volatile WaitCtl* abortp = &wait_ctl;
+  // A launch this small takes a few microseconds, of which getting started is a good part: it is launched
+  // with programmatic stream serialisation, so that on idle SMs the next one has set up when this one ends
+  if (kHalves) {
+    grid_dependency_wait();
+    grid_launch_dependents();
+  }
 
   // kHalves: row maximum and row sum of a slot's keys, [item & 1][slot][row]; it has no use for the staging buffer
   float2* row_stat = reinterpret_cast<float2*>(smem_raw + (sO - raw));
@@ -1416,9 +1422,10 @@ int launch(const TyrAttnPrefillArgs& a, float scale, int* status, cudaStream_t s
     return (int)cudaGetLastError();
   }
   if (halves) {
-    prefill_kernel<D, kNoMask, false, false, true><<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, p, to);
+    cudaError_t e = launch_overlapped(prefill_kernel<D, kNoMask, false, false, true>, dim3(grid), dim3(kThreads), C::kSmemBytes,
+                                      st, 1, tq, tk, tv, to, p, to);
     count_launch();
-    return (int)cudaGetLastError();
+    return (int)(e != cudaSuccess ? e : cudaGetLastError());
   }
   prefill_kernel<D, kMask, false, false, false><<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, p, to);
   count_launch();
