@@ -457,8 +457,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   auto bar = [&](int i) { return sBar + 8u * i; };
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // the merge kernel behind a split launch may become resident as SMs fall free (it waits for this grid itself)
-  if (kSplit) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int total_items = p.items_per_group * p.n_kv_head * p.batch + (kSplit ? p.n_split * (p.n_parts - 1) : 0);
 
   if (threadIdx.x == 0) {
@@ -480,12 +478,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
   volatile WaitCtl* abortp = &wait_ctl;
-  // A launch this small takes a few microseconds, of which getting started is a good part: it is launched
-  // with programmatic stream serialisation, so that on idle SMs the next one has set up when this one ends
-  if (kHalves) {
-    grid_dependency_wait();
-    grid_launch_dependents();
-  }
+  // A short launch is made with programmatic stream serialisation (overlaps_predecessor): on SMs that are idle
+  // or fall free it has set up when the one before ends.  A no-op in other launches.
+  grid_dependency_wait();
+  grid_launch_dependents();
 
   // kHalves: row maximum and row sum of a slot's keys, [item & 1][slot][row]; it has no use for the staging buffer
   float2* row_stat = reinterpret_cast<float2*>(smem_raw + (sO - raw));
@@ -1162,7 +1158,8 @@ bool halves_pay(const TyrAttnPrefillArgs& a, int n_sm) {
 // Tyr/GPU/Kernels/RingAttn.lean:164-180 over the parts of a split item.  16 bytes of a row per lane.
 template <int D>
 __global__ void __launch_bounds__(256) prefill_split_merge_kernel(const PrefillParams p) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  grid_dependency_wait();
+  grid_launch_dependents();
   constexpr int kLanesPerRow = D / 8;            // 16 bytes of a row per lane
   constexpr int kRowsPerWarp = 32 / kLanesPerRow;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1277,6 +1274,20 @@ bool item_table_for(PrefillParams& p, int grid, cudaStream_t st) {
   return true;
 }
 
+// Launches of up to this many KV-tile steps per CTA (about 75 us) overlap the one before them: that saves 1.5 to 4 us
+// (2.6 rounds of 1 to 2 tiles, forward of 64 x 6 heads of 256 x 64 with its backward: 78.4 -> 77.0; 216 items of 18 tiles
+// with the split of the last round: 65.9 -> 62.2; 700 rows with a window of 256 and 3 padded prompts of 200 rows:
+// 16.4 -> 16.1 and 14.4).  In longer ones the CTAs' places on the SMs, then in the order in which these fall free,
+// cost more than that: 8 x 2048 rows 150 -> 154 us, 4 x 8192 1853 -> 1907.
+constexpr int kOverlapSteps = 40;
+bool overlaps_predecessor(const PrefillParams& p, long long items, int n_sm) {
+  const int nkv = (p.kv_seq + kBN - 1) / kBN, rows = p.pair_heads ? kBM : 2 * kBM;
+  long long tiles = nkv;  // of an average item
+  if (p.causal) tiles = std::min<long long>(tiles, ((long long)p.n_mblk * rows / kBN + 1) / 2);
+  if (p.window > 0) tiles = std::min<long long>(tiles, (p.window + rows + kBN - 1) / kBN);
+  return items * tiles <= (long long)kOverlapSteps * n_sm;
+}
+
 template <int D, int kMask>
 int launch(const TyrAttnPrefillArgs& a, float scale, int* status, cudaStream_t st) {
   using C = Cfg<D>;
@@ -1371,6 +1382,7 @@ int launch(const TyrAttnPrefillArgs& a, float scale, int* status, cudaStream_t s
   p.wait_limit = wait_limit_cycles();
   const long long items = (long long)p.items_per_group * a.n_kv_head * a.batch;
   if (items > 0x7fffffffLL) return -TYR_ATTN_ERR_TOO_LARGE;
+  const bool overlap = overlaps_predecessor(p, items, sm_count());
   p.split_from = (int)items;
   p.n_split = 0;
   p.n_parts = 1;
@@ -1390,22 +1402,14 @@ int launch(const TyrAttnPrefillArgs& a, float scale, int* status, cudaStream_t s
     const int64_t part_stride[3] = {2ll * kBM * D, (int64_t)kBM * D, D};
     if ((rc = make_map(&top, p.o_part, sp.n_parts * sp.n_split, 2, kBM, D, part_stride))) return rc;
     const int grid = (int)std::min<long long>(items + (long long)sp.n_split * (sp.n_parts - 1), sm_count());
-    prefill_kernel<D, kNoMask, true, false, false><<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, p, top);
+    cudaError_t e = launch_kernel(prefill_kernel<D, kNoMask, true, false, false>, dim3(grid), dim3(kThreads), C::kSmemBytes, st, 1,
+                                  overlap, tq, tk, tv, to, p, top);
     count_launch();
-    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return (int)e;
     // programmatic stream serialisation: the merge's launch latency hides behind the kernel's tail
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(sp.n_split * 256 / (8 * (32 / (D / 8))));   // 256 rows per item, 8 warps of 32 / (D / 8) rows
-    cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, prefill_split_merge_kernel<D>, p);
+    const unsigned merge_ctas = sp.n_split * 256 / (8 * (32 / (D / 8)));   // 256 rows per item, 8 warps of 32 / (D / 8) rows
+    e = launch_overlapped(prefill_split_merge_kernel<D>, dim3(merge_ctas), dim3(256), 0, st, 1, p);
     count_launch();
     if (e == cudaSuccess) e = cudaGetLastError();
     return (int)e;
@@ -1417,9 +1421,10 @@ int launch(const TyrAttnPrefillArgs& a, float scale, int* status, cudaStream_t s
   // (and not for launches so large that the table itself would weigh: 4 bytes and a heap step per item)
   if (kMask == kNoMask && D == 128 && p.causal && !p.snake && items >= 4ll * grid && items <= kMaxTabledItems &&
       item_table_for(p, grid, st)) {
-    prefill_kernel<128, kNoMask, false, true, false><<<grid, kThreads, Cfg<128>::kSmemBytes, st>>>(tq, tk, tv, to, p, to);
+    cudaError_t e = launch_kernel(prefill_kernel<128, kNoMask, false, true, false>, dim3(grid), dim3(kThreads),
+                                  Cfg<128>::kSmemBytes, st, 1, overlap, tq, tk, tv, to, p, to);
     count_launch();
-    return (int)cudaGetLastError();
+    return (int)(e != cudaSuccess ? e : cudaGetLastError());
   }
   if (halves) {
     cudaError_t e = launch_overlapped(prefill_kernel<D, kNoMask, false, false, true>, dim3(grid), dim3(kThreads), C::kSmemBytes,
@@ -1427,9 +1432,10 @@ int launch(const TyrAttnPrefillArgs& a, float scale, int* status, cudaStream_t s
     count_launch();
     return (int)(e != cudaSuccess ? e : cudaGetLastError());
   }
-  prefill_kernel<D, kMask, false, false, false><<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, p, to);
+  cudaError_t e = launch_kernel(prefill_kernel<D, kMask, false, false, false>, dim3(grid), dim3(kThreads), C::kSmemBytes, st, 1,
+                                overlap, tq, tk, tv, to, p, to);
   count_launch();
-  return (int)cudaGetLastError();
+  return (int)(e != cudaSuccess ? e : cudaGetLastError());
 }
 
 }  // namespace
