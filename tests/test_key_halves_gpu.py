@@ -38,3 +38,15 @@ def test_few_items(B, Hq, Hkv, Sq, Skv, causal, D):
     ro, rlse = c_oracle.sdpa(q.float().numpy(), k.float().numpy(), v.float().numpy(), causal)
     assert np.abs(o.float().cpu().numpy() - ro).max() <= O_MAX_ABS
     assert (np.abs(lse.cpu().numpy() - rlse) / np.maximum(np.abs(rlse), 1.0)).max() <= LSE_REL
+
+
+# windows shorter than a tile, of a few tiles and longer than the prompt: rows to which a slot's tiles show no key
+@pytest.mark.parametrize("S,window", [(700, 1), (700, 100), (700, 256), (1023, 300), (1500, 130), (385, 1000)])
+@pytest.mark.parametrize("Hq,Hkv", [(16, 4), (5, 5)])
+@pytest.mark.parametrize("D", [64, 128])
+def test_few_items_under_a_window(S, window, Hq, Hkv, D):
+    q, k, v = randn(1, Hq, S, D, seed=S), randn(1, Hkv, S, D, seed=S + 1), randn(1, Hkv, S, D, seed=S + 2)
+    o, lse = tnn.attentionFwd(q.to(DEV), k.to(DEV), v.to(DEV), window_size=window)
+    ro, rlse = c_oracle.sdpa(q.float().numpy(), k.float().numpy(), v.float().numpy(), True, window=window)
+    assert np.abs(o.float().cpu().numpy() - ro).max() <= O_MAX_ABS
+    assert (np.abs(lse.cpu().numpy() - rlse) / np.maximum(np.abs(rlse), 1.0)).max() <= LSE_REL

@@ -239,8 +239,8 @@ __device__ __forceinline__ Item decode_item(int w, const PrefillParams& p) {
   if (kHalves) {
     it.hq[0] = it.hq[1] = it.hkv * p.group + hl;
     it.row[0] = it.row[1] = it.mblk * kBM;
-    const int n = p.causal ? min(nkv_total, it.mblk + 1) : nkv_total;
-    it.lo = 0;
+    it.lo = (kMask != kNoMask && p.window > 0) ? max(0, it.row[0] - p.window + 1) / kBN : 0;
+    const int n = (p.causal ? min(nkv_total, it.mblk + 1) : nkv_total) - it.lo;
     it.n0 = (n + 1) >> 1;  // tiles 0, 2, ..
     it.n1 = n >> 1;        // tiles 1, 3, ..
     return it;
@@ -1138,15 +1138,18 @@ SplitPlan split_plan(const TyrAttnPrefillArgs& a, int n_sm) {
 // launch of at most one round of work items, whose time is that of its longest item, when the CTA with the
 // most work then has less.  In halves of a KV-tile step, an item boundary counted as one, with the merge as
 // two.  One prompt of 517 rows, 32 heads of 128: 80 items of up to 5 steps become 160 of up to 3, 16.4 ->
-// 14.4 us; 1024 rows, 16 heads 22.5 -> 16.4 us; 40 rows on 700 keys 17.2 -> 12.3 us.
+// 14.4 us; 1024 rows, 16 heads 22.5 -> 16.4 us; 40 rows on 700 keys 17.2 -> 12.3 us; with a window of 64,
+// 2 x 500 rows, 12 heads of 64 12.1 -> 8.0 us, of 1000, 1000 rows, 6 heads of 64 18.0 -> 11.7 us.
 bool halves_pay(const TyrAttnPrefillArgs& a, int n_sm) {
-  if (a.window_size > 0 || a.key_mask != nullptr) return false;
+  if (a.key_mask != nullptr) return false;
   const int nkv = (a.kv_seq + kBN - 1) / kBN, n_mblk = (a.q_seq + kBM - 1) / kBM;
   const long long per_level = (long long)a.n_head * a.batch, items = per_level * n_mblk;
   if (a.q_seq >= kOneOrderSeq || a.kv_seq >= kOneOrderSeq) return false;
   if (items > 2ll * n_sm || split_plan(a, n_sm).items > n_sm) return false;
   auto tiles = [&](long long w) {  // KV tiles of item w, longest first
-    return a.is_causal ? std::min<int>(nkv, n_mblk - (int)(w / per_level)) : nkv;
+    const int mblk = n_mblk - 1 - (int)(w / per_level);
+    const int lo = a.window_size > 0 ? std::max(0, mblk * kBM - a.window_size + 1) / kBN : 0;
+    return (a.is_causal || a.window_size > 0 ? std::min<int>(nkv, mblk + 1) : nkv) - lo;
   };
   auto cost = [&](long long w) { return 2 * ((tiles(w) + 1) / 2) + 2; };
   int busiest = cost(0);
@@ -1312,8 +1315,8 @@ int launch(const TyrAttnPrefillArgs& a, float scale, int* status, cudaStream_t s
                                         (int)C::kSmemBytes);
         if (attr_err != cudaSuccess) return (int)attr_err;
       }
-      if (kMask == kNoMask) {
-        attr_err = cudaFuncSetAttribute(prefill_kernel<D, kNoMask, false, false, true>,
+      if constexpr (kMask != kKeyMask) {
+        attr_err = cudaFuncSetAttribute(prefill_kernel<D, kMask, false, false, true>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmemBytes);
         if (attr_err != cudaSuccess) return (int)attr_err;
       }
@@ -1338,7 +1341,7 @@ int launch(const TyrAttnPrefillArgs& a, float scale, int* status, cudaStream_t s
     sp = split_plan(a, sm_count());
     if (a.workspace_bytes < sp.bytes || (reinterpret_cast<uintptr_t>(a.workspace) & 255) != 0) sp.n_split = 0;
   }
-  const bool halves = kMask == kNoMask && sp.n_split == 0 &&
+  const bool halves = kMask != kKeyMask && sp.n_split == 0 &&
                       4ll * a.kv_seq * D * a.batch * a.n_kv_head <= kOneChunkBytes && halves_pay(a, sm_count());
   {
     const int group = a.n_head / a.n_kv_head;
@@ -1426,11 +1429,13 @@ int launch(const TyrAttnPrefillArgs& a, float scale, int* status, cudaStream_t s
     count_launch();
     return (int)(e != cudaSuccess ? e : cudaGetLastError());
   }
-  if (halves) {
-    cudaError_t e = launch_overlapped(prefill_kernel<D, kNoMask, false, false, true>, dim3(grid), dim3(kThreads), C::kSmemBytes,
-                                      st, 1, tq, tk, tv, to, p, to);
-    count_launch();
-    return (int)(e != cudaSuccess ? e : cudaGetLastError());
+  if constexpr (kMask != kKeyMask) {
+    if (halves) {
+      cudaError_t e = launch_overlapped(prefill_kernel<D, kMask, false, false, true>, dim3(grid), dim3(kThreads), C::kSmemBytes,
+                                        st, 1, tq, tk, tv, to, p, to);
+      count_launch();
+      return (int)(e != cudaSuccess ? e : cudaGetLastError());
+    }
   }
   cudaError_t e = launch_kernel(prefill_kernel<D, kMask, false, false, false>, dim3(grid), dim3(kThreads), C::kSmemBytes, st, 1,
                                 overlap, tq, tk, tv, to, p, to);
