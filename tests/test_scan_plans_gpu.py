@@ -5,7 +5,7 @@ import torch
 
 from conftest import LSE_REL, O_MAX_ABS
 from oracle import c_oracle
-from tyr_b200 import nn as tnn
+from tyr_b200 import _lib, nn as tnn
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -66,3 +66,27 @@ def test_few_query_rows(Hq, Hkv, Sq, workspace):
     buf = torch.full((2, Sq, Hq, D), 7.0, dtype=torch.bfloat16, device=DEV)     # [B,S,H,D] storage on both sides
     o, lse = tnn.attentionFwd(q.to(DEV), k.to(DEV), v.to(DEV), is_causal=False, out=buf.transpose(1, 2), workspace=workspace)
     check(o, lse, q, k, v)
+
+
+# calls that no workspace helps: more (sequence, KV head) pairs than one wave of CTAs has slots, long keys without a workspace
+# or with one that is too small; the output starts as a value that no attention over these V gives
+@pytest.mark.parametrize("B,Hq,Hkv,L,D,workspace", [
+    (40, 32, 8, 1100, 128, None), (13, 24, 24, 1500, 128, None), (25, 12, 12, 3000, 64, None), (50, 6, 6, 2049, 64, None),
+    (1, 32, 8, 20000, 128, False), (4, 24, 24, 2000, 128, False), (17, 32, 8, 2051, 128, False), (4, 24, 24, 2000, 128, "small")])
+def test_typed_call_without_a_usable_workspace(B, Hq, Hkv, L, D, workspace):
+    q, k, v = randn(B, Hq, 1, D, seed=L), randn(B, Hkv, L, D, seed=L + 1), randn(B, Hkv, L, D, seed=L + 2)
+    dev = [t.to(DEV) for t in (q, k, v)]
+    out = torch.full((B, Hq, 1, D), 77.0, dtype=torch.bfloat16, device=DEV)
+    if workspace == "small":
+        assert tnn.prefill_workspace_bytes(*dev, is_causal=False) > 256
+        workspace = torch.empty(256, dtype=torch.uint8, device=DEV)
+    n0 = tnn.launch_count()
+    o, lse = tnn.attentionFwd(*dev, is_causal=False, out=out, workspace=workspace)
+    assert tnn.launch_count() - n0 == 1
+    rows = sorted({0, B // 2, B - 1})     # the oracle's share
+    check(o[rows], lse[rows], q[rows], k[rows], v[rows])
+    raw = torch.full_like(out, 77.0)      # the C entry that mirrors the reference's extern: it has no workspace argument
+    _lib.check(_lib.load().tyr_b200_sdpa_gqa_qkv(B, Hq, Hkv, 1, L, D, *(t.data_ptr() for t in dev), raw.data_ptr(), 0.0, 0, 1,
+                                                 torch.cuda.current_stream().cuda_stream))
+    check(raw[rows], None, q[rows], k[rows], v[rows])
+    assert not (o == 77.0).any() and not (raw == 77.0).any()

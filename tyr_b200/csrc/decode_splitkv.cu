@@ -33,11 +33,11 @@
 #include "attn_internal.h"
 #include "mma_sync.cuh"
 #include "ptx_sm100.cuh"
+#include "scan_plan.h"
 
 namespace tyr {
 namespace {
 
-constexpr int kWarpKeys = 16;   // keys of a pipeline stage one warp works on
 constexpr int kStages = 3;
 constexpr int kMergeThreads = 128;
 constexpr int kMaxFewRows = 16;
@@ -492,12 +492,6 @@ cudaError_t launch_scan(const DecodeParams& p, cudaStream_t st) {
                            kSmem, st, kCluster ? p.n_splits : 1, p);
 }
 
-// How a launch cuts its keys.
-struct ScanPlan {
-  bool cluster;   // n_splits CTAs per (sequence, KV head, row group) merge among themselves; else chunk_len keys per CTA
-  int n_splits, chunk_len, warps;
-};
-
 template <int D, int kNT>
 cudaError_t launch_scan_of(const DecodeParams& p, const ScanPlan& s, cudaStream_t st) {
   if (s.cluster) return s.warps == 8 ? launch_scan<D, 8, kNT, true>(p, st) : launch_scan<D, 4, kNT, true>(p, st);
@@ -506,51 +500,20 @@ cudaError_t launch_scan_of(const DecodeParams& p, const ScanPlan& s, cudaStream_
 
 template <int D>
 int launch_d(DecodeParams& p, const ScanPlan& s, cudaStream_t st) {
+  if (!s.covers(p.max_kv_seq)) return -TYR_ATTN_ERR_SHAPE;  // (the kernel divides by the chunk length)
   p.n_splits = s.n_splits;
   p.chunk_len = s.chunk_len;
   cudaError_t e = p.rows <= 8 ? launch_scan_of<D, 1>(p, s, st) : launch_scan_of<D, 2>(p, s, st);
   count_launch();
   if (e != cudaSuccess) return (int)e;
-  if (!s.cluster && p.n_splits > 1) {
+  if (s.needs_workspace()) {
     e = launch_overlapped(decode_merge_kernel<D>, dim3(p.n_head * p.q_seq, p.batch), dim3(kMergeThreads), 0, st, 1, p);
     count_launch();
   }
   return (int)(e != cudaSuccess ? e : cudaGetLastError());
 }
 
-constexpr int kChunkUnit = 64;  // keys; chunk lengths are multiples of it
-
-// The cut of a launch small enough to be done without a workspace: one chunk per (sequence, KV head), or a
-// cluster of CTAs for each.  `units`: (sequence, KV head, row group) triples.  Returns false for launches
-// that a cut into chunks of the workspace form serves better.
-//
-// The most CTAs that still run all at once, clusters placed: two per SM less the slots a GPC cannot
-// give to whole clusters.  Clusters of 16 leave more of them unused and are only taken where half the
-// slots are enough (for head_dim 64 three quarters).  A CTA gets at least one step of its warps' keys (64 or 128); past
-// 1024 (head_dim 64: 2048) keys per CTA the workspace form's greater choice of chunk counts wins.
-// Device time, workspace form -> this one, 8 KV heads of 128: one sequence of 512 keys 8.2 -> 4.8 us,
-// 1537: 8.8 -> 6.7, 4096: 9.5 -> 8.5, 16384: 18.9 -> 18.3 (32768: 29.2 -> 30.7, not taken); 4 x 2051 12.6 -> 10.8,
-// 4 x 8192 27.1 -> 24.2; 8 x 1537 14.2 -> 13.2; 12 KV heads of 64: 1537 7.1 -> 5.4, 4 x 8192 23.7 -> 20.0.
-// Eight warps per CTA instead of four where one CTA has an SM to itself, and for head_dim 64, whose
-// stages are half as large.
-bool small_scan_plan(int head_dim, long long units, int max_len, int max_splits, ScanPlan* s) {
-  const int sm = sm_count(), slots = 2 * sm - sm / 4;
-  const int warps = head_dim == 64 ? 8 : 4;
-  int n = (int)std::min<long long>(8, slots / std::max<long long>(units, 1));
-  if (units * 16 <= (head_dim == 64 ? slots * 3 / 4 : slots / 2)) n = 16;
-  n = std::min(n, (max_len + kWarpKeys * warps - 1) / (kWarpKeys * warps));
-  n = std::max(std::min(n, max_splits), 1);
-  if (max_len > (head_dim == 64 ? 2048 : 1024) * n) return false;
-  // few, long pieces that leave a quarter of the slots empty (4 x 24 KV heads, 2000 keys: 29.2 against 25.7 us)
-  if (n > 1 && n < 8 && max_len > 512 * n && units * n * 4 < slots * 3) return false;
-  s->cluster = n > 1;
-  s->n_splits = n;
-  s->chunk_len = n > 1 ? 0 : (max_len + kChunkUnit - 1) / kChunkUnit * kChunkUnit;
-  s->warps = n > 1 ? warps : (units <= sm ? 8 : 4);
-  return true;
-}
-
-int max_splits_of(int max_splits) { return max_splits <= 0 || max_splits > 64 ? 64 : max_splits; }
+int max_splits_of(int max_splits) { return max_splits <= 0 || max_splits > kMaxWsChunks ? kMaxWsChunks : max_splits; }
 
 }  // namespace
 
@@ -647,7 +610,7 @@ int launch_decode(const TyrAttnDecodeArgs& a, float scale, cudaStream_t st) {
     if (!ds) return -TYR_ATTN_ERR_NO_DEVICE;
     p.status = ds->status;
   }
-  ScanPlan s{false, 1, 0, 4};
+  ScanPlan s;
   s.n_splits = decode_launch_splits(a.max_kv_seq, a.max_splits, a.batch, a.n_kv_head * p.row_groups,
                                     a.total_kv_len > 0 ? a.total_kv_len : 0, a.kv_lens == nullptr || a.total_kv_len > 0,
                                     &s.chunk_len);
@@ -658,36 +621,20 @@ int launch_decode(const TyrAttnDecodeArgs& a, float scale, cudaStream_t st) {
     p.ws_lse = p.ws_o + (size_t)a.batch * a.n_head * s.n_splits * a.head_dim;
     p.ws_aligned = (reinterpret_cast<uintptr_t>(p.ws_o) & 15) == 0;
   }
-  small_scan_plan(a.head_dim, (long long)a.batch * a.n_kv_head * p.row_groups, a.max_kv_seq, max_splits_of(a.max_splits), &s);
+  bool pays;
+  const ScanPlan own = own_scan_plan(a.head_dim, (long long)a.batch * a.n_kv_head * p.row_groups, a.max_kv_seq,
+                                     max_splits_of(a.max_splits), sm_count(), &pays);
+  if (pays) s = own;
   if (a.head_dim == 128) return launch_d<128>(p, s, st);
   if (a.head_dim == 64) return launch_d<64>(p, s, st);
   return -TYR_ATTN_ERR_HEAD_DIM;
 }
 
 // ---- the typed call with few query rows per KV head
-namespace {
-
-ScanPlan few_rows_plan(const TyrAttnPrefillArgs& a, bool have_workspace) {
+static ScanPlan few_rows_plan_of(const TyrAttnPrefillArgs& a, bool have_workspace) {
   const int rows = a.n_head / a.n_kv_head * a.q_seq;
-  const long long units = (long long)a.batch * a.n_kv_head * ((rows + 15) / 16);
-  ScanPlan s{false, 1, 0, 4};
-  const bool small = small_scan_plan(a.head_dim, units, a.kv_seq, 64, &s);
-  // One or two (batch, KV head) pairs over at least 1024 keys keep to the workspace where the caller gives
-  // one, as such calls always have: it reaches more of the device than two clusters of 16 can (one
-  // sequence of 16384 keys, two KV heads: 12.5 us against 13.2; of 1500 keys 6.8 against 4.7).
-  if (!have_workspace || (small && !(units <= 2 && a.kv_seq >= 1024))) return s;
-  // chunks that give one wave of CTAs, as in decode_launch_splits
-  const int slots = 2 * sm_count();
-  long long c = ((long long)a.kv_seq * units + slots - 1) / slots;
-  c = std::max<long long>(c, (a.kv_seq + 63) / 64);
-  s.cluster = false;
-  s.warps = 4;
-  s.chunk_len = (int)((c + kChunkUnit - 1) / kChunkUnit * kChunkUnit);
-  s.n_splits = (a.kv_seq + s.chunk_len - 1) / s.chunk_len;
-  return s;
+  return few_rows_plan(a.head_dim, (long long)a.batch * a.n_kv_head * ((rows + 15) / 16), a.kv_seq, have_workspace, sm_count());
 }
-
-}  // namespace
 
 bool few_rows_call(const TyrAttnPrefillArgs& a) {
   return !a.is_causal && a.window_size == 0 && a.key_mask == nullptr && !a.check_mode && a.dtype == TYR_ATTN_BF16 &&
@@ -695,8 +642,8 @@ bool few_rows_call(const TyrAttnPrefillArgs& a) {
 }
 
 size_t few_rows_workspace_bytes(const TyrAttnPrefillArgs& a) {
-  const ScanPlan s = few_rows_plan(a, true);
-  if (s.cluster || s.n_splits <= 1) return 0;
+  const ScanPlan s = few_rows_plan_of(a, true);
+  if (!s.needs_workspace()) return 0;
   return (size_t)a.batch * a.n_head * a.q_seq * s.n_splits * ((size_t)a.head_dim + 1) * sizeof(float);
 }
 
@@ -720,7 +667,7 @@ int launch_few_rows(const TyrAttnPrefillArgs& a, float scale, int* status, cudaS
   const size_t need = few_rows_workspace_bytes(a);
   const bool ws = a.workspace != nullptr && need > 0 && (size_t)a.workspace_bytes >= need &&
                   (reinterpret_cast<uintptr_t>(a.workspace) & 255) == 0;
-  const ScanPlan s = few_rows_plan(a, ws);
+  const ScanPlan s = few_rows_plan_of(a, ws);
   p.ws_o = static_cast<float*>(a.workspace);
   p.ws_lse = ws ? p.ws_o + (size_t)a.batch * a.n_head * a.q_seq * s.n_splits * a.head_dim : nullptr;
   p.ws_aligned = 1;
