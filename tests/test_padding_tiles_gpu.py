@@ -54,3 +54,26 @@ def test_padding_mask_cuts_tiles(Hq, Hkv, S, window, causal, D):
     assert np.nanmax(np.abs(o - ro)) <= O_MAX_ABS
     some = np.isfinite(rlse)
     assert (np.abs(lse[some] - rlse[some]) / np.maximum(np.abs(rlse[some]), 1.0)).max() <= LSE_REL
+
+
+# one mask for the whole batch, a window moving over one buffer, a transposed mask, a slice of a wider one: a mask of any
+# strides gives the bits of its contiguous copy
+@pytest.mark.parametrize("dtype", [torch.bool, torch.uint8, torch.int64, torch.float32])
+@pytest.mark.parametrize("causal", [False, True])
+def test_masks_of_any_strides(dtype, causal):
+    B, H, S, D = 3, 4, 300, 64
+    q, k, v = (randn(B, H, S, D, seed=s).to(DEV) for s in (1, 2, 3))
+    bits = torch.rand(2000, generator=torch.Generator().manual_seed(4)) < 0.6
+    bits[0] = bits[:S] = True       # every causal row has a key
+    line = bits.to(DEV).to(dtype)
+    wide = line[:B * 400].view(B, 400)
+    masks = [line[40:40 + S][None].expand(B, S), line[None, :S].expand(B, -1), line.as_strided((B, S), (7, 1)),
+             line[:S * B].view(S, B).t(), wide[:, :S], wide[:1, :S].expand(B, S), line[:2 * S].as_strided((B, S), (0, 2))]
+    for m in masks:
+        want = tnn.scaledDotProductAttentionGQAMask(q, k, v, m.ne(0).clone(memory_format=torch.contiguous_format), 0.0, causal)
+        got = tnn.scaledDotProductAttentionGQAMask(q, k, v, m, 0.0, causal)
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.nan_to_num(), want.nan_to_num())
+    with pytest.raises(ValueError):
+        tnn.scaledDotProductAttentionGQAMask(q, k, v, line[0], 0.0, causal)
+    with pytest.raises(ValueError):
+        tnn.scaledDotProductAttentionGQAMask(q, k, v, line[:S], 0.0, causal)

@@ -169,8 +169,10 @@ def scaledDotProductAttentionGQAMask(query, key, value, attn_mask, dropout_p: fl
         raise AttnError(-2)
     if query.shape[2] != key.shape[2]:
         raise ValueError("scaledDotProductAttentionGQAMask needs q_seq == kv_seq")
-    km = attn_mask        # one byte per key for the C ABI
-    if km.dtype not in (torch.bool, torch.uint8) or km.stride(-1) != 1:
+    # one byte per key for the C ABI, the rows of a batch apart: a byte mask goes as it is, anything else (another type,
+    # a mask shared by the batch through `expand`, overlapping rows) as a copy
+    km = attn_mask
+    if km.dtype not in (torch.bool, torch.uint8) or km.dim() != 2 or km.stride(1) != 1 or km.stride(0) < km.shape[1]:
         km = (km != 0).contiguous()
     out, _ = attentionFwd(query, key, value, is_causal=is_causal, return_lse=False, key_mask=km)
     return out
