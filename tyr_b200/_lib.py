@@ -148,7 +148,8 @@ def calls():
     import torch  # noqa: F401  (its libraries have to be loaded first)
     load()
     if not os.path.exists(CALLS_PATH):
-        raise ImportError(f"{CALLS_PATH} is missing: run `python -c 'import __graft_entry__ as g; g.build()'`")
+        raise ImportError(f"{CALLS_PATH} is missing: run `python -c 'import __graft_entry__ as g; g.build()'` "
+                          "where g++ and a torch with CUDA are installed")
     spec = importlib.util.spec_from_file_location("_calls", CALLS_PATH)
     mod = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(mod)

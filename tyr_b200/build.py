@@ -4,6 +4,8 @@ from __future__ import annotations
 import os
 import shutil
 import subprocess
+import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -39,15 +41,19 @@ def _older(path: str, deps) -> bool:
     return any(os.path.getmtime(os.path.join(CSRC, d)) > t for d in deps)
 
 
-def stale() -> bool:
-    return _older(LIB_PATH, SOURCES + HEADERS) or _older(CALLS_PATH, [CALLS_SOURCE, HEADERS[-1]])
+def library_stale() -> bool:
+    return _older(LIB_PATH, SOURCES + HEADERS)
 
 
 def _calls_command():
-    """g++ command of the call layer.  It sees the C ABI's header only and is linked against the library next to it."""
-    import sysconfig
-
-    import torch
+    """g++ command of the call layer.  It sees the C ABI's header only and is linked against the library next to it.
+    None where it cannot be built: the C ABI needs neither g++ nor a torch with CUDA, the Python calls need both."""
+    try:
+        import torch
+    except ImportError:
+        return None
+    if torch.version.cuda is None or shutil.which("g++") is None:
+        return None
     root = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(nvcc_path()))
     return (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
@@ -58,19 +64,46 @@ def _calls_command():
              "-ltorch_cuda", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"])
 
 
+def _calls_stamp() -> str:
+    """What the call layer's binary interface depends on beside its sources."""
+    import torch
+    return f"python {sys.version}\ntorch {torch.__version__} {torch.version.git_version}\n"
+
+
+def calls_stale() -> bool:
+    """The call layer is missing, older than its sources, or built for another Python or torch (and can be built)."""
+    if _calls_command() is None:
+        return False
+    if _older(CALLS_PATH, [CALLS_SOURCE, HEADERS[-1]]) or not os.path.exists(CALLS_PATH + ".built_for"):
+        return True
+    with open(CALLS_PATH + ".built_for") as f:
+        return f.read() != _calls_stamp()
+
+
+def stale() -> bool:
+    return library_stale() or calls_stale()
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Build lib/libtyr_b200_attn.so if missing or older than its sources."""
-    if not force and not stale():
-        return LIB_PATH
+    """Build lib/libtyr_b200_attn.so, and the Python call layer where it can be built, if missing or stale."""
     os.makedirs(LIB_DIR, exist_ok=True)
-    cmd = [nvcc_path()] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else [])
-    cmd += ["-o", LIB_PATH] + [os.path.join(CSRC, f) for f in SOURCES]
-    for c in ([cmd] if force or _older(LIB_PATH, SOURCES + HEADERS) else []) + [_calls_command()]:
-        res = subprocess.run(c, capture_output=True, text=True)
+
+    def run(cmd):
+        res = subprocess.run(cmd, capture_output=True, text=True)
         if verbose:
             print(res.stderr)
         if res.returncode != 0:
-            raise RuntimeError(os.path.basename(c[0]) + " failed:\n" + res.stderr)
+            raise RuntimeError(os.path.basename(cmd[0]) + " failed:\n" + res.stderr)
+
+    if force or library_stale():
+        run([nvcc_path()] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) +
+            ["-o", LIB_PATH] + [os.path.join(CSRC, f) for f in SOURCES])
+    if force or calls_stale():
+        cmd = _calls_command()
+        if cmd is not None:
+            run(cmd)
+            with open(CALLS_PATH + ".built_for", "w") as f:
+                f.write(_calls_stamp())
     return LIB_PATH
 
 
