@@ -72,3 +72,32 @@ def test_dq_written_over_an_input(over):
         a.dtype, a.is_causal, a.scale, a.workspace_bytes = _lib.TYR_ATTN_BF16, 1, 0.0, ws.numel() * 4
         _lib.check(lib.tyr_b200_attn_backward(ctypes.byref(a), torch.cuda.current_stream().cuda_stream))
         assert all(torch.equal(x, y) for x, y in zip((t[over], d_k, d_v), want))
+
+
+@pytest.mark.parametrize("B,H,S", [(1, 4, 700), (4, 12, 1500)])     # clusters of the dK/dV kernel, and one CTA a unit
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("D", [64, 128])
+def test_steps_on_one_workspace(B, H, S, masked, D):
+    # a training loop: row statistics and mask change from step to step at the same addresses, and the dQ kernel runs next
+    # to the dK/dV kernel; every step has the bits of a call of its own
+    q, k, v = (randn(B, H, S, D, seed=s).to(DEV) for s in (1, 2, 3))
+    d_o = [randn(B, H, S, D, seed=10 + i).to(DEV) * (1 + i) for i in range(6)]
+    masks = [None] * 6
+    if masked:
+        masks = [(torch.arange(S) < S - 90 * i).to(torch.uint8).expand(B, S).contiguous().to(DEV) for i in range(6)]
+    alone = []
+    for g, m in zip(d_o, masks):
+        o, lse = tnn.attentionFwd(q, k, v, key_mask=m)
+        torch.cuda.synchronize()
+        alone.append((o, lse) + tnn.attentionBwd(q, k, v, o, lse, g, key_mask=m))
+        torch.cuda.synchronize()
+    ws = torch.empty(_lib.load().tyr_b200_attn_backward_workspace_bytes(B, H, S) // 4, device=DEV)
+    m = None if masks[0] is None else masks[0].clone()
+    for _ in range(3):
+        got = []
+        for i, g in enumerate(d_o):
+            if m is not None:
+                m.copy_(masks[i])
+            got.append(tnn.attentionBwd(q, k, v, alone[i][0], alone[i][1], g, workspace=ws, key_mask=m))
+        for x, y in zip(got, alone):
+            assert all(torch.equal(a, b) for a, b in zip(x, y[2:]))

@@ -13,7 +13,7 @@ namespace tyr {
 // griddepcontrol.wait (grid_dependency_wait) in every thread block before it touches memory that an
 // earlier grid may write or still read, so only its launch latency and set-up overlap.  A grid lets
 // its successor start by griddepcontrol.launch_dependents (grid_launch_dependents).  The one exception
-// is the dQ kernel of the backward, which runs next to the dK/dV kernel and waits for it at its end.
+// is the dQ kernel of the backward, which runs next to the dK/dV kernel, reads its inputs from L2 and waits at its end.
 template <class... P, class... A>
 inline cudaError_t launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, unsigned cluster_x,
                                  bool overlap, A&&... args) {

@@ -249,8 +249,10 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
   const uint32_t tmem = tmem_slot;
   volatile WaitCtl* abortp = &wait_ctl;
   // the row statistics (and everything before them in the stream) are complete from here on; the dQ kernel,
-  // which needs nothing of this one, may take the SMs that this one leaves or does not fill
+  // which needs nothing of this one, may take the SMs that this one leaves or does not fill.  It does not wait for
+  // that grid itself, so every thread fences between what the wait has made visible to it and the release.
   grid_dependency_wait();
+  __threadfence();
   grid_launch_dependents();
 
   if (warp == 0) {
@@ -735,8 +737,11 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
   volatile WaitCtl* abortp = &wait_ctl;
-  // Every CTA of the grid before has passed its own wait for the row statistics: the inputs are complete.  That
-  // grid may still be running and reading the inputs, so an output that overlaps one of them waits.
+  // Every CTA of the grid before has passed its own wait for the row statistics: the inputs are complete, in L2.  Without a
+  // wait nothing says that this SM's L1 holds no older lines of them (the statistics and often the mask lie at the
+  // same addresses in every step of a training loop), so all of them come from L2: the tiles by TMA, the row
+  // statistics and mask bytes by ld_gpu_*.  The grid before may still be running and reading the inputs, so an
+  // output that overlaps one of them waits.
   if (p.wait_first) grid_dependency_wait();
 
   if (warp == 0) {
@@ -842,7 +847,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       const QUnit w = q_unit(u, p);
       const int row0 = w.blk * kT;
       const int64_t at = ((int64_t)w.b * p.n_head + w.head) * p.sq_pad + row0 + r;
-      const float nl_row = p.neg_lse2[at], nd_row = p.neg_delta_s[at];
+      const float nl_row = ld_gpu_f32(p.neg_lse2 + at), nd_row = ld_gpu_f32(p.neg_delta_s + at);
       const uint64_t nl2 = pack_f32x2(nl_row, nl_row), nd2 = pack_f32x2(nd_row, nd_row);
       for (int i = 0; i < w.n_iter; ++i, ++it) {
         ok = mbar_wait_q(bar(C::s_full), it & 1, abortp);
@@ -878,7 +883,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             const int kk = 2 * lane + e;
-            vb[e] = __ballot_sync(0xffffffffu, (col0 + 64 * half + kk < p.kv_seq) && mrow[kk] != 0);
+            vb[e] = __ballot_sync(0xffffffffu, (col0 + 64 * half + kk < p.kv_seq) && ld_gpu_u8(mrow + kk) != 0);
           }
         }
         const bool masked = __any_sync(0xffffffffu, c_limit < kT || c_first > 0) || (vb[0] & vb[1]) != 0xffffffffu;

@@ -23,6 +23,18 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 // See launch_overlapped (attn_internal.h).
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Loads from L2, the point of coherence, whatever this SM's L1 holds: for a kernel that runs next to the grid before
+// it and reads what earlier grids have written without a griddepcontrol.wait of its own.
+__device__ __forceinline__ float ld_gpu_f32(const float* p) {
+  float v;
+  asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint32_t ld_gpu_u8(const uint8_t* p) {
+  uint32_t v;
+  asm volatile("ld.relaxed.gpu.global.u8 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
 
 // --------------------------------------------------------- thread-block cluster
 __device__ __forceinline__ void cluster_sync() {
