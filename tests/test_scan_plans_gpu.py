@@ -90,3 +90,31 @@ def test_typed_call_without_a_usable_workspace(B, Hq, Hkv, L, D, workspace):
                                                  torch.cuda.current_stream().cuda_stream))
     check(raw[rows], None, q[rows], k[rows], v[rows])
     assert not (o == 77.0).any() and not (raw == 77.0).any()
+
+
+# Keys whose score is -inf (a K row with -inf where the query has a positive entry), as many as a warp's 16, a tile's 64, a
+# CTA's and a chunk's share of the keys and a KV tile of 128, at the start, in the middle and at the end: such keys have no
+# weight, however they are cut.  Cluster (640 keys, 5 pairs), one chunk (700 pairs), workspace (24 and 2 pairs, long).
+@pytest.mark.parametrize("B,Hq,Hkv,L", [(1, 10, 5, 640), (100, 7, 7, 300), (1, 24, 24, 9000), (1, 4, 2, 20000)])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("dense", [False, True])
+def test_scores_of_minus_infinity(B, Hq, Hkv, L, D, dense):
+    q, k, v = randn(B, Hq, 1, D, seed=L), randn(B, Hkv, L, D, seed=L + 1), randn(B, Hkv, L, D, seed=L + 2)
+    q[..., 0] = 1.0
+    hidden = torch.zeros(L, dtype=torch.bool)
+    for at, n in ((0, 128), (144, 16), (192, 64), (L // 2, L // 5), (L - 40, 40)):
+        hidden[at:at + n] = True
+    seen = (~hidden).nonzero()[:, 0]
+    k[:, :, hidden, 0] = -torch.inf
+    if dense:
+        o, lse = tnn.flashDecodeDense(q.to(DEV), k.to(DEV), v.to(DEV))
+        o, lse = o[:, :, None], lse[:, :, None]
+    else:
+        o, lse = tnn.attentionFwd(q.to(DEV), k.to(DEV), v.to(DEV), is_causal=False)
+    rows = [0, B - 1]
+    check(o[rows], lse[rows], q[rows], k[rows][:, :, seen], v[rows][:, :, seen])
+    assert not o.isnan().any()
+    # no key at all: NaN, as from ATen
+    k[..., 0] = -torch.inf
+    o, _ = tnn.attentionFwd(q.to(DEV), k.to(DEV), v.to(DEV), is_causal=False)
+    assert o.isnan().all()

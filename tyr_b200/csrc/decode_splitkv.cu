@@ -76,6 +76,11 @@ __device__ __forceinline__ int64_t lse_index(const DecodeParams& p, int b, int h
   return (int64_t)b * p.n_head * p.q_seq + hkv * p.rows + r;
 }
 
+// The value scores are taken relative to, given their maximum so far.  Where all of them are -inf that is 0, so that
+// their exponentials and the weight of what was summed before are 0 and not 2^(-inf + inf): a warp sees 16 keys
+// at a time, and a key whose products with the query overflow to -inf, or that a caller masks that way, has no weight.
+__device__ __forceinline__ float finite_ref(float m) { return m == -INFINITY ? 0.f : m; }
+
 // A length outside [1, max_kv_seq] (the workspace and the grid are sized for max_kv_seq, so a
 // longer one would index past both): report it once per sequence, give a sequence without any
 // key a defined row (zeros, LSE = -inf), and return the length forced into [0, max_kv_seq].
@@ -256,8 +261,8 @@ decode_kernel(const __grid_constant__ DecodeParams p) {
         float alpha[2];
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
-          const float m_new = fmaxf(m_run[nt][x], mx[nt][x]);  // finite: key gkey0 is valid
-          alpha[x] = ex2f(m_run[nt][x] - m_new);               // 0 on the first tile
+          const float m_new = fmaxf(m_run[nt][x], mx[nt][x]);
+          alpha[x] = ex2f(m_run[nt][x] - finite_ref(m_new));   // 0 on the first tile
           m_run[nt][x] = m_new;
           l_run[nt][x] *= alpha[x];
         }
@@ -274,8 +279,9 @@ decode_kernel(const __grid_constant__ DecodeParams p) {
     uint32_t pb[kNT][2];
 #pragma unroll
     for (int nt = 0; nt < kNT; ++nt) {
-      const float p0 = ex2f(sx[nt][0] - m_run[nt][0]), p1 = ex2f(sx[nt][1] - m_run[nt][1]);
-      const float p2 = ex2f(sx[nt][2] - m_run[nt][0]), p3 = ex2f(sx[nt][3] - m_run[nt][1]);
+      const float m0 = finite_ref(m_run[nt][0]), m1 = finite_ref(m_run[nt][1]);
+      const float p0 = ex2f(sx[nt][0] - m0), p1 = ex2f(sx[nt][1] - m1);
+      const float p2 = ex2f(sx[nt][2] - m0), p3 = ex2f(sx[nt][3] - m1);
       l_run[nt][0] += p0 + p2;
       l_run[nt][1] += p1 + p3;
       pb[nt][0] = transpose_8x8(pack2(p0, p1));
@@ -343,7 +349,8 @@ decode_kernel(const __grid_constant__ DecodeParams p) {
       }
       continue;
     }
-    const float outv = acc / L;
+    // L = 0: every score is -inf.  Of the whole sequence that gives NaN, as from ATen; a chunk of it has no weight.
+    const float outv = (n_chunks > 1 && L == 0.f) ? 0.f : acc / L;
     const float lse2 = M + log2f(L);
     if (n_chunks == 1) {
       o_row(p, b, hkv, row0 + r)[d] = __float2bfloat16_rn(outv);
@@ -375,13 +382,13 @@ decode_kernel(const __grid_constant__ DecodeParams p) {
         float m_new = M;
 #pragma unroll
         for (int c = 0; c < 8; ++c) m_new = fmaxf(m_new, m8[c]);
-        const float f0 = ex2f(M - m_new);
+        const float ref = finite_ref(m_new), f0 = ex2f(M - ref);
         L *= f0;
         acc *= f0;
         M = m_new;
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-          const float f = c0 + c < n_chunks ? ex2f(m8[c] - M) : 0.f;
+          const float f = c0 + c < n_chunks ? ex2f(m8[c] - ref) : 0.f;
           L = fmaf(l8[c], f, L);
           acc = fmaf(a8[c], f, acc);
         }
