@@ -77,3 +77,22 @@ def test_masks_of_any_strides(dtype, causal):
         tnn.scaledDotProductAttentionGQAMask(q, k, v, line[0], 0.0, causal)
     with pytest.raises(ValueError):
         tnn.scaledDotProductAttentionGQAMask(q, k, v, line[:S], 0.0, causal)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_mask_rewritten_between_calls(D):
+    # short masked launches overlap the one before them, which here writes the mask: each call sees its own mask
+    B, H, S = 4, 6, 500
+    q, k, v = (randn(B, H, S, D, seed=s).to(DEV) for s in (1, 2, 3))
+    masks = [(torch.arange(S) < S - 60 * i).to(torch.uint8).expand(B, S).contiguous().to(DEV) for i in range(8)]
+    alone = []
+    for m in masks:
+        alone.append(tnn.attentionFwd(q, k, v, key_mask=m))
+        torch.cuda.synchronize()
+    m = torch.empty_like(masks[0])
+    for _ in range(5):
+        got = []
+        for x in masks:
+            m.copy_(x)
+            got.append(tnn.attentionFwd(q, k, v, key_mask=m))
+        assert all(torch.equal(a, b) for x, y in zip(got, alone) for a, b in zip(x, y))

@@ -11,7 +11,8 @@ namespace tyr {
 // Launch with programmatic stream serialisation: the kernel's CTAs may become resident while the
 // grid before it in the stream is still draining.  Every kernel launched this way executes
 // griddepcontrol.wait (grid_dependency_wait) in every thread block before it touches memory that an
-// earlier grid may write or still read, so only its launch latency and set-up overlap.  A grid lets
+// earlier grid may write or still read, so only its launch latency and set-up overlap (and reads such memory by ordinary
+// loads: the read-only path is for what no one writes during a kernel's lifetime, which begins earlier here).  A grid lets
 // its successor start by griddepcontrol.launch_dependents (grid_launch_dependents).  The one exception
 // is the dQ kernel of the backward, which runs next to the dK/dV kernel, reads its inputs from L2 and waits at its end.
 template <class... P, class... A>

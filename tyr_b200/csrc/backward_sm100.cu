@@ -973,11 +973,12 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 }
 
 // Row statistics of the backward: one group of D/8 lanes per query row, 16-byte loads.
+// (The pointers are not __restrict__: its CTAs are resident while the grid before may still be writing O, dO and the
+// LSE, which rules the read-only path out.)
 template <int D>
 __global__ void __launch_bounds__(256)
-bwd_rowstats_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                    const float* __restrict__ lse, float* __restrict__ neg_lse2,
-                    float* __restrict__ neg_delta_s, int n_head, int q_seq, int sq_pad, int64_t os_b,
+bwd_rowstats_kernel(const __nv_bfloat16* o, const __nv_bfloat16* d_o, const float* lse, float* neg_lse2,
+                    float* neg_delta_s, int n_head, int q_seq, int sq_pad, int64_t os_b,
                     int64_t os_h, int64_t os_s, int64_t ds_b, int64_t ds_h, int64_t ds_s, float scale,
                     int64_t total_rows) {
   constexpr int kLanes = D / 8;  // lanes per row

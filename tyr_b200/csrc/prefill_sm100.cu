@@ -311,6 +311,8 @@ __device__ __forceinline__ Item work_item(int w, const PrefillParams& p) {
 // Returns the item's (lo, n0, n1) cut down to those between them; each Q tile keeps at least one KV tile (a
 // batch row without a valid key in reach: its rows come out as NaN, as from ATen).  Looks at four tiles at a
 // time from either end, so a batch row padded on one side takes a round or two per end.
+// (Ordinary loads of the mask here and in the softmax warps: a launch that overlaps the one before is resident while that
+// one may still be writing the mask, which rules the read-only path out.)
 // Not inlined: its registers would be the kernel's (scores of a whole row are live elsewhere).
 // The masked launches are bound like the others by softmax and tensor pipe, so a tile not visited is time saved,
 // and the look-up runs on an idle warp two items ahead.  With the mask bytes fetched before the wait for the
@@ -326,7 +328,7 @@ __device__ __noinline__ int4 valid_tiles(const uint8_t* mrow, int kv_seq, int lo
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const int kk = (j0 + x) * kBN + c * 32 + lane;
-        if (j0 + x >= lo && j0 + x < end && kk < kv_seq) v[x] |= __ldg(mrow + kk);
+        if (j0 + x >= lo && j0 + x < end && kk < kv_seq) v[x] |= mrow[kk];
       }
 #pragma unroll
     for (int x = 0; x < 4; ++x) any |= (__any_sync(0xffffffffu, v[x] != 0u) ? 1u : 0u) << x;
@@ -791,7 +793,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           const uint8_t* mrow = p.key_mask + im.b * p.key_mask_stride + kk;
 #pragma unroll
           for (int c = 0; c < 4; ++c)
-            if (kk + 32 * c < p.kv_seq && __ldg(mrow + 32 * c) != 0) valid4 |= 1u << c;
+            if (kk + 32 * c < p.kv_seq && mrow[32 * c] != 0) valid4 |= 1u << c;
         }
         ok = mbar_wait(bar(B::s_full + t), sc & 1, abortp);
         ok = __all_sync(0xffffffffu, ok);
