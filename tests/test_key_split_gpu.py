@@ -30,7 +30,7 @@ def _close_to_unsplit(q, k, v, o, lse):
 
 
 @pytest.mark.parametrize("D", [64, 128])
-@pytest.mark.parametrize("Sq,Skv", [(2048, 2048), (300, 2000), (128, 1024), (1, 1500), (200, 1100)])
+@pytest.mark.parametrize("Sq,Skv", [(2048, 2048), (300, 2000), (128, 1024), (1, 20000), (200, 1100)])
 def test_single_round_is_split_and_matches_the_oracle(D, Sq, Skv):
     q, k, v = randn(1, 4, Sq, D, seed=Sq + D), randn(1, 2, Skv, D, seed=Skv + 1), randn(1, 2, Skv, D, seed=Skv + 2)
     qd, kd, vd = q.to(DEV), k.to(DEV), v.to(DEV)

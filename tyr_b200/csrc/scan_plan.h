@@ -58,10 +58,12 @@ inline ScanPlan own_scan_plan(int head_dim, long long units, int max_len, int ma
 inline ScanPlan few_rows_plan(int head_dim, long long units, int kv_seq, bool have_workspace, int sm) {
   bool pays;
   const ScanPlan own = own_scan_plan(head_dim, units, kv_seq, kMaxWsChunks, sm, &pays);
-  // One or two (batch, KV head) pairs over at least 1024 keys keep to the workspace where the caller gives
-  // one, as such calls always have: it reaches more of the device than two clusters of 16 can (one
-  // sequence of 16384 keys, two KV heads: 12.5 us against 13.2; of 1500 keys 6.8 against 4.7).
-  if (!have_workspace || (pays && !(units <= 2 && kv_seq >= 1024))) return own;
+  // One or two (batch, KV head) pairs over long keys: chunks in the workspace reach more of the device than one or two
+  // clusters of 16 can, and cost a second launch.  Workspace form against clusters, one pair: heads of 64 6000 keys 7.3
+  // against 6.9 us, 8192 7.3 / 7.5, 16384 8.3 / 10.0; of 128 8192 10.6 / 9.6, 12000 11.4 / 11.8, 16384 11.8 / 14.1; two pairs:
+  // of 64 8192 7.7 / 7.5, 12000 8.1 / 8.7; of 128 12000 12.4 / 12.0, 16384 13.2 / 14.3.
+  const bool long_pair = units <= 2 && kv_seq > (head_dim == 64 ? 8192 : 12288);
+  if (!have_workspace || (pays && !long_pair)) return own;
   // chunks that give one wave of CTAs, as in decode_launch_splits
   const int slots = 2 * sm;
   long long c = ((long long)kv_seq * units + slots - 1) / slots;
