@@ -46,6 +46,7 @@
 
 #include "attn_internal.h"
 #include "ptx_sm100.cuh"
+#include "unit_parts.h"
 
 namespace tyr {
 namespace {
@@ -1013,35 +1014,45 @@ bwd_rowstats_kernel(const __nv_bfloat16* o, const __nv_bfloat16* d_o, const floa
   }
 }
 
-// CTAs that share a unit of the dK/dV kernel.  A launch of few units takes as long as its longest one (the
-// first keys are seen by every query row of every head of the group); several CTAs per unit cost a
-// cluster's merge and a CTA's set-up each, together about kMergePairs streamed pairs.  The number with the
-// shortest time, taken as the longest unit or the average load of the clusters that run at once, and only
-// where it is a tenth shorter.  One prompt of 512 rows, 32/8 heads: 32 units on 148 SMs; forward and backward
-// 53 -> 41 us at D = 128, 43 -> 33 us at D = 64.
-constexpr int kMergePairs = 3;
-int unit_parts(const BwdParams& p, int sms) {
-  const long long units = (long long)p.n_kblk * p.n_kv_head * p.batch;
-  if (units >= 2ll * sms || p.q_seq >= kOneOrderSeq || p.kv_seq >= kOneOrderSeq) return 1;
-  long long best = 0;
-  int best_parts = 1;
-  for (int parts = 1; parts <= 8; parts *= 2) {
-    long long longest = 0, total = 0;
-    for (int blk = 0; blk < p.n_kblk; ++blk) {
-      const int lo = p.causal ? std::min(blk, p.n_qblk) : 0;
-      const int hi = p.window > 0 ? std::min(p.n_qblk, (blk * kT + kT - 1 + p.window - 1) / kT + 1) : p.n_qblk;
-      const long long n = (long long)std::max(hi - lo, 0) * p.group;
-      const long long cost = (n + parts - 1) / parts + (parts > 1 ? kMergePairs : 1);
-      longest = std::max(longest, cost);
-      total += cost * p.n_kv_head * p.batch;
+// CTAs that share a unit of the dK/dV kernel (unit_parts.h).  How many clusters run at once depends on how the SMs are
+// spread over the GPCs: asked for once per device.
+template <int D>
+int unit_parts(const BwdParams& p, int dev, int sms) {
+  static std::atomic<int> known[64][kPartsChoices] = {};  // per device; 0: not asked yet, else capacity + 1
+  if ((long long)p.n_kblk * p.n_kv_head * p.batch >= 2ll * sms || p.q_seq >= kOneOrderSeq || p.kv_seq >= kOneOrderSeq) return 1;
+  int capacity[kPartsChoices] = {sms, 0, 0, 0};
+  for (int k = 1; k < kPartsChoices; ++k) {
+    int c = known[dev][k].load(std::memory_order_relaxed);
+    if (c == 0) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(1u << k);
+      cfg.blockDim = dim3(kBwdThreads);
+      cfg.dynamicSmemBytes = BCfg<D>::kSmemBytes;
+      cudaLaunchAttribute attr;
+      attr.id = cudaLaunchAttributeClusterDimension;
+      attr.val.clusterDim.x = 1u << k;
+      attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+      cfg.attrs = &attr;
+      cfg.numAttrs = 1;
+      int n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, bwd_dkdv_kernel<D, true>, &cfg) != cudaSuccess) {
+        cudaGetLastError();  // no clusters of this size then
+        n = 0;
+      }
+      c = n + 1;
+      known[dev][k].store(c, std::memory_order_relaxed);
     }
-    const long long span = std::max(longest, total * parts / sms);
-    if (parts == 1 || 10 * span < 9 * best) {
-      best = span;
-      best_parts = parts;
-    }
+    capacity[k] = c - 1;
   }
-  return best_parts;
+  BwdSizes z;
+  z.n_kblk = p.n_kblk;
+  z.n_qblk = p.n_qblk;
+  z.n_kv = p.n_kv_head * p.batch;
+  z.n_q = p.n_head * p.batch;
+  z.group = p.group;
+  z.window = p.window;
+  z.causal = p.causal != 0;
+  return choose_unit_parts(z, sms, capacity);
 }
 
 template <int D>
@@ -1059,9 +1070,9 @@ int launch_bwd(const TyrAttnBackwardArgs& a, float scale, int* status, cudaStrea
   if ((rc = make_tile_map(&tk, a.k, a.batch, a.n_kv_head, a.kv_seq, D, a.k_stride))) return rc;
   if ((rc = make_tile_map(&tv, a.v, a.batch, a.n_kv_head, a.kv_seq, D, a.v_stride))) return rc;
   if ((rc = make_tile_map(&tdo, a.d_o, a.batch, a.n_head, a.q_seq, D, a.do_stride))) return rc;
+  int dev = 0;
   {
     static std::atomic<bool> attr_set[64] = {};
-    int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -TYR_ATTN_ERR_NO_DEVICE;
     if (!attr_set[dev].load(std::memory_order_acquire)) {
       cudaError_t e = cudaFuncSetAttribute(bwd_dkdv_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1129,7 +1140,7 @@ int launch_bwd(const TyrAttnBackwardArgs& a, float scale, int* status, cudaStrea
     p.out2_stride[i] = a.dv_stride[i];
   }
   p.wait_first = 0;
-  p.parts = unit_parts(p, sms);
+  p.parts = unit_parts<D>(p, dev, sms);
   cudaError_t e = p.parts > 1
                       ? launch_overlapped(bwd_dkdv_kernel<D, true>, dim3((unsigned)(grid_kv * p.parts)), dim3(kBwdThreads),
                                           C::kSmemBytes, st, (unsigned)p.parts, tk, tv, tq, tdo, p)
