@@ -1279,18 +1279,22 @@ bool item_table_for(PrefillParams& p, int grid, cudaStream_t st) {
   return true;
 }
 
-// Launches of up to this many KV-tile steps per CTA (about 75 us) overlap the one before them: that saves 1.5 to 4 us
-// (2.6 rounds of 1 to 2 tiles, forward of 64 x 6 heads of 256 x 64 with its backward: 78.4 -> 77.0; 216 items of 18 tiles
-// with the split of the last round: 65.9 -> 62.2; 700 rows with a window of 256 and 3 padded prompts of 200 rows:
+// Launches of up to a number of KV-tile steps per CTA overlap the one before them: that saves 1.5 to 4 us (216 items of 18
+// tiles with the split of the last round: 65.9 -> 62.2; 700 rows with a window of 256 and 3 padded prompts of 200 rows:
 // 16.4 -> 16.1 and 14.4).  In longer ones the CTAs' places on the SMs, then in the order in which these fall free,
-// cost more than that: 8 x 2048 rows 150 -> 154 us, 4 x 8192 1853 -> 1907.
-constexpr int kOverlapSteps = 40;
-bool overlaps_predecessor(const PrefillParams& p, long long items, int n_sm) {
+// cost more than that (8 x 2048 rows 150 -> 154 us, 4 x 8192 1853 -> 1907), and the sooner the more a wrong place costs:
+//  * items of one length, and heads of 64: 40 steps.  59 of 59 measured launches of up to 38 steps gain (0.4 to 15 %).
+//  * heads of 128, items of unequal length (causal, window): two heads an item 18 (48 of 53 launches below gain, up to 13 %,
+//    16 of 24 above lose, up to 5.7 %: 13 x 636 rows, 32/8 heads 64.2 -> 66.7), 20 under a padding mask, whose tiles without a key
+//    shorten the items (8 x 1111 rows, 16/8 heads: 65.2 -> 64.0); one head an item 28 (54 of 55 below gain, up to 11 %, 10 of
+//    17 above lose, up to 4.4 %: 59 x 336 rows, 24 heads 142.9 -> 149.2).
+bool overlaps_predecessor(const PrefillParams& p, int head_dim, long long items, int n_sm) {
   const int nkv = (p.kv_seq + kBN - 1) / kBN, rows = p.pair_heads ? kBM : 2 * kBM;
   long long tiles = nkv;  // of an average item
   if (p.causal) tiles = std::min<long long>(tiles, ((long long)p.n_mblk * rows / kBN + 1) / 2);
   if (p.window > 0) tiles = std::min<long long>(tiles, (p.window + rows + kBN - 1) / kBN);
-  return items * tiles <= (long long)kOverlapSteps * n_sm;
+  const int steps = head_dim == 64 || !p.causal ? 40 : !p.pair_heads ? 28 : p.key_mask != nullptr ? 20 : 18;
+  return items * tiles <= (long long)steps * n_sm;
 }
 
 template <int D, int kMask>
@@ -1387,7 +1391,7 @@ int launch(const TyrAttnPrefillArgs& a, float scale, int* status, cudaStream_t s
   p.wait_limit = wait_limit_cycles();
   const long long items = (long long)p.items_per_group * a.n_kv_head * a.batch;
   if (items > 0x7fffffffLL) return -TYR_ATTN_ERR_TOO_LARGE;
-  const bool overlap = overlaps_predecessor(p, items, sm_count());
+  const bool overlap = overlaps_predecessor(p, D, items, sm_count());
   p.split_from = (int)items;
   p.n_split = 0;
   p.n_parts = 1;
