@@ -251,10 +251,14 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant_
   volatile WaitCtl* abortp = &wait_ctl;
   // the row statistics (and everything before them in the stream) are complete from here on; the dQ kernel,
   // which needs nothing of this one, may take the SMs that this one leaves or does not fill.  It does not wait for
-  // that grid itself, so every thread fences between what the wait has made visible to it and the release.
+  // that grid itself, so a fence lies between what the wait has made visible here and the release, both by one
+  // thread (with a fence in every thread 4 x 8 heads of 200 rows x 128 take 14.64 us instead of 14.45).
   grid_dependency_wait();
-  __threadfence();
-  grid_launch_dependents();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    grid_launch_dependents();
+  }
+  __syncwarp();
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
