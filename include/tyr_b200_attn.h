@@ -94,18 +94,25 @@ typedef struct TyrAttnPrefillArgs {
   int64_t key_mask_stride; /* bytes between the mask rows of two batch elements */
   void* workspace;         /* NULL, or DEVICE scratch of tyr_b200_attn_prefill_workspace_bytes(args)
                               bytes, 256-byte aligned, private to this call until it has finished on
-                              its stream.  With it a non-causal launch whose last round of work items
-                              fills at most half the SMs computes that round's items in two to eight
-                              parts of their keys and merges them (Tyr/GPU/Kernels/RingAttn.lean:164-180).
-                              Without it, or when it is too small, nothing is split. */
+                              its stream.  With it an unmasked non-causal launch whose last round of
+                              work items fills at most half the SMs computes that round's items in two to
+                              eight parts of their keys and merges them (Tyr/GPU/Kernels/RingAttn.lean:164-180),
+                              and one with at most 16 query rows per KV head (n_head / n_kv_head * q_seq)
+                              over long keys cuts them into chunks and merges those.  Without it, or when
+                              it is too small, the call is one launch: the former is not split, the latter
+                              leaves a KV head's keys to one CTA or to a cluster of up to 16. */
   int64_t workspace_bytes;
 } TyrAttnPrefillArgs;
 
+/* Order of sums: every call gives the same bits each time.  A causal or windowed forward or backward
+ * with q_seq >= 2048 or kv_seq >= 2048 also gives each batch element the bits of a call of its own.
+ * Below that, and in other calls, the cut of a row's keys (or a key's rows) depends on the number of
+ * work items of the whole launch, so a batch element agrees with a call of its own to rounding. */
 int tyr_b200_attn_prefill(const TyrAttnPrefillArgs* args, void* stream);
-/* Bytes of `workspace` with which the call above would split its last round on the current
- * device; 0 when it would not split (causal, windowed or masked calls, short key sequences, a
- * last round that is more than half full, more than eight full rounds before it), negative
- * TYR_ATTN_ERR_* on bad arguments. */
+/* Bytes of `workspace` that the call above would use on the current device; 0 when it would use
+ * none (causal, windowed or masked calls, short key sequences, a last round that is more than half
+ * full, more than eight full rounds before it, few query rows whose keys one wave of CTAs holds
+ * uncut or in clusters), negative TYR_ATTN_ERR_* on bad arguments. */
 int64_t tyr_b200_attn_prefill_workspace_bytes(const TyrAttnPrefillArgs* args);
 
 /* Contiguous-layout forms whose argument lists mirror the Lean externs one to

@@ -85,15 +85,15 @@ def attentionFwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, is_causal: b
     Launcher convention of Examples/GPU/RunFlashAttn.lean:68-81: outputs may be
     pre-allocated by the caller and are written in place.
     `workspace`: a caller-kept uint8 CUDA tensor of `prefill_workspace_bytes(...)` bytes for the
-    key-split of a half-empty last round; when the call would split, one is allocated if none is given
-    (`workspace=False`: never split).
+    key-split of a half-empty last round, or of long keys under few query rows; when the call would use
+    one, it is allocated if none is given (`workspace=False`: one launch without any).
     """
     return _lib.calls().attention_fwd(q, k, v, is_causal, scale, out, lse, return_lse, check_mode, window_size,
                                       key_mask, workspace)
 
 
 def prefill_workspace_bytes(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, is_causal: bool = True) -> int:
-    """Bytes of `workspace` with which `attentionFwd` on these tensors would split its last round (0: it would not)."""
+    """Bytes of `workspace` that `attentionFwd` on these tensors would use (0: none)."""
     a = _fill_prefill(q, k, v, q, None, is_causal, None, False)  # only shapes and strides are looked at
     with torch.cuda.device(q.device):
         return max(int(_lib.load().tyr_b200_attn_prefill_workspace_bytes(ctypes.byref(a))), 0)
