@@ -24,7 +24,8 @@ def _status_clean():
 
 
 # one KV tile (slot 1 idle), two, an odd and an even number, tails of one row and one key, a second round of items on
-# some CTAs (160, 200 and 264 items on 148 SMs), one query row block against several tiles, 32 tiles (the longest)
+# some CTAs (160, 200 and 264 items on 148 SMs), one query row block against several tiles; 4096 rows, which keep the
+# plain form (one order of sums from 2048 on)
 @pytest.mark.parametrize("B,Hq,Hkv,Sq,Skv,causal", [
     (1, 8, 2, 129, 129, True), (1, 8, 2, 256, 256, True), (1, 4, 4, 385, 385, True), (1, 32, 8, 517, 517, True),
     (1, 25, 5, 1023, 1023, True), (2, 12, 12, 1400, 1400, True), (1, 2, 1, 4096, 4096, True), (1, 8, 8, 300, 300, False),

@@ -35,7 +35,7 @@
 // output columns.  Units are sorted by decreasing work and dealt to the CTAs in mirrored rounds.
 // The three launches overlap (launch_overlapped): each sets up while the one before drains, and the dQ kernel,
 // which needs the row statistics only, takes every SM that the dK/dV kernel leaves or does not fill.  64 x 6
-// heads of 256 rows x 64: 65.9 -> 59.2 us; one prompt of 512 rows, 32/8 heads of 128, with its forward 69 -> 53 us.
+// heads of 256 rows x 64: 65.9 -> 59.2 us; one prompt of 512 rows, 32/8 heads of 128, with its forward 69 -> 54 us.
 // Every wait is bounded and reports through the per-device status word, as in the forward.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -86,8 +86,8 @@ struct BCfg {
   static constexpr int p_half = kB + 13;               // kHalfP: P^T of query columns 0..63 written (8 warp arrivals)
   static constexpr int kNumBars = kB + 14;
   // D = 128: P^T is handed over in two halves, so that dV of the first 64 query columns runs during the
-  // exponentials of the second 64.  The backward of 4096 rows, 32/8 heads 405.3 -> 399.0 us, of 8 x 2048 rows,
-  // 16/8 heads 487.3 -> 484.3; at D = 64, where the elementwise warps are the bound, the extra hand-over cost 0.3 %.
+  // exponentials of the second 64.  The backward of 4096 rows, 32/8 heads 396.7 -> 391.9 us, of 8 x 2048 rows,
+  // 16/8 heads 480.3 -> 477.8, of 2304 rows x 24 heads without a mask 185.6 -> 183.4; at D = 64, where the elementwise warps are the bound, the extra hand-over cost 0.3 %.
   static constexpr bool kHalfP = (D == 128);
   static constexpr uint32_t kSmemBytes = kBarOff + kNumBars * 8 + 16 + 1024;  // + align slack
   static constexpr uint32_t kTmemCols = 512;

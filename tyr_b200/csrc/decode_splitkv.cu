@@ -161,7 +161,7 @@ decode_kernel(const __grid_constant__ DecodeParams p) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int quad = lane >> 2, t4 = lane & 3;
 
-  // ---- stage loader: 64 keys x D bf16 of K and of V, 16 bytes per cp.async
+  // ---- stage loader: kTileKeys keys x D bf16 of K and of V, 16 bytes per cp.async
   auto load_tile = [&](int tile, int stage) {
     const uint32_t sk = sbase + stage * C::kStageBytes, sv = sk + C::kTileBytes;
     const int k0 = key_begin + tile * kTileKeys;

@@ -4,9 +4,9 @@
 //
 // A single-token step or a short prompt is a few microseconds of device work, and building the
 // argument structures from Python cost 14 to 38 us per call (ctypes fields, a device context
-// manager, tensor attributes one by one): the host set the pace.  Host time of a pass, before -> after:
-// three prologues and a dense decode 84 -> 31 us, the typed call on a 517-row prompt 30 -> 7 us, forward
-// and backward 74 -> 25 us; the passes that were bound by it, queued back to back: 75 -> 34, 22 -> 16 us.
+// manager, tensor attributes one by one): the host set the pace.  Host time of a pass with the GPU idle, before ->
+// after: three prologues and a dense decode 79 -> 23 us, the typed call on a 517-row prompt 21 -> 5.5 us, forward and
+// backward 81 -> 18 us, a single-row typed call 35 -> 9.5 us.
 // Nothing is cached here: every call reads its tensors anew.
 //
 // The Python functions keep names, defaults and results; they hand their arguments over by position.
@@ -112,7 +112,7 @@ Tensor new_tensor(at::IntArrayRef size, at::ScalarType dt, at::Device dev) {
 }
 void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
 
-// `mask` as one byte per key for the C ABI; may allocate (and launch) when its type is not a byte already
+// The mask as the C ABI takes it, one byte per key; checked only, other types are converted by the Python caller.
 Tensor key_bytes(const Tensor& m, int64_t batch, int64_t kv_seq) {
   const bool byte = m.scalar_type() == at::kBool || m.scalar_type() == at::kByte;
   if (!m.is_cuda() || !byte || m.dim() != 2 || m.stride(1) != 1 || m.size(0) != batch || m.size(1) != kv_seq)
