@@ -51,3 +51,21 @@ def test_few_items_under_a_window(S, window, Hq, Hkv, D):
     ro, rlse = c_oracle.sdpa(q.float().numpy(), k.float().numpy(), v.float().numpy(), True, window=window)
     assert np.abs(o.float().cpu().numpy() - ro).max() <= O_MAX_ABS
     assert (np.abs(lse.cpu().numpy() - rlse) / np.maximum(np.abs(rlse), 1.0)).max() <= LSE_REL
+
+
+# From 2048 query rows or keys on a batch element of a causal or windowed call has the bits of a call of its own, forward
+# and backward, although the launch of the one has too few work items for the SMs and that of the other has not
+@pytest.mark.parametrize("Sq,Skv,window", [(2048, 2048, 0), (2100, 2100, 200), (300, 2048, 0), (2048, 300, 0)])
+@pytest.mark.parametrize("D", [64, 128])
+def test_one_order_of_sums_for_long_calls(Sq, Skv, window, D):
+    B, Hq, Hkv = 7, 4, 2
+    q, d_o = randn(B, Hq, Sq, D, seed=Sq).to(DEV), randn(B, Hq, Sq, D, seed=Sq + 1).to(DEV)
+    k, v = randn(B, Hkv, Skv, D, seed=Skv + 2).to(DEV), randn(B, Hkv, Skv, D, seed=Skv + 3).to(DEV)
+
+    def both(*t):
+        o, lse = tnn.attentionFwd(*t[:3], window_size=window)
+        return (o, lse) + tnn.attentionBwd(*t[:3], o, lse, t[3], window_size=window)
+    whole = both(q, k, v, d_o)
+    for b in (0, B - 1):
+        one = both(*(t[b:b + 1] for t in (q, k, v, d_o)))
+        assert all(torch.equal(x[b:b + 1], y) for x, y in zip(whole, one))
