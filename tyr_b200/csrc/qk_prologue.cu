@@ -168,9 +168,19 @@ prologue_kernel(const PrologueParams p) {
 // of 2048 tokens 6.2 -> 5.3 us.  The pair form's 2x2 table is as many bytes as a token's two heads in and
 // out and each CTA reads it again, so that form keeps as many heads as leave 256 CTAs (32 heads of 16 K
 // tokens: 47.5 us with all of them, 55.1 with four; of 2048 tokens: 17.0 with all, 8.9 with eight).
-int heads_per_cta(int n_head, int64_t token_blocks, bool pairs) {
+// The other form's tables are read again by every group of heads too, from L2 only while they stay there: the groups
+// follow one another over all tokens. Where a group's rows in and out are more than L2 (126 MB), or the tables more than
+// 12 MB, a CTA does all heads of its tokens: against the groups 2 x 32768 tokens, 16 heads of 128 102.3 -> 91.7 us, 3 x 20000, 12
+// heads of 256 144.0 -> 125; at 4 x 16384, 12 heads of 128 (134 MB) 68.9 -> 69.8, at 2 x 16384 (67 MB) 37.0 -> 39.0. A last group of
+// one to three heads reads a table row for little data, and loses sooner: 34 x 4141 tokens, 5 heads of 64 43.9 -> 40.1,
+// 15 x 4266 (62 MB) 20.6 -> 19.5, 9 x 4266 (37 MB) 13.6 -> 13.4; 7 heads 23.9 -> 24.1 and 14.2 -> 14.3 there.
+int heads_per_cta(int n_head, int64_t token_blocks, bool pairs, int64_t group_bytes, int64_t table_bytes) {
   int h = (n_head + kHeadsInFlight - 1) / kHeadsInFlight * kHeadsInFlight;
-  if (!pairs) return kHeadsInFlight;
+  if (!pairs) {
+    const bool spilled = table_bytes > (12ll << 20) || group_bytes > ((n_head % kHeadsInFlight == 0 ? 128ll : 48ll) << 20);
+    if (n_head > 65535 * kHeadsInFlight) return h;  // (the grid's y extent)
+    return table_bytes > 0 && spilled ? h : kHeadsInFlight;
+  }
   while (h > kHeadsInFlight && token_blocks * ((n_head + h - 1) / h) < 256)
     h = (h / 2 + kHeadsInFlight - 1) / kHeadsInFlight * kHeadsInFlight;
   return h;
@@ -206,7 +216,8 @@ int launch_qk_prologue(const TyrAttnPrologueArgs& a, int* status, cudaStream_t s
   const int tok_per_block = kWarps * (512 / a.head_dim);
   const int64_t blocks = (tokens + tok_per_block - 1) / tok_per_block;
   if (blocks > 0x7fffffffLL) return -TYR_ATTN_ERR_TOO_LARGE;
-  p.heads_per_cta = heads_per_cta(a.n_head, blocks, a.pe != nullptr);
+  p.heads_per_cta = heads_per_cta(a.n_head, blocks, a.pe != nullptr, tokens * a.head_dim * 4 * kHeadsInFlight,
+                                  a.cos != nullptr ? (int64_t)a.seq * a.head_dim * 4 : 0);
   const dim3 grid((unsigned)blocks, (a.n_head + p.heads_per_cta - 1) / p.heads_per_cta);
   int rc;
   if (a.head_dim == 128) rc = launch_d<128>(p, grid, st);
